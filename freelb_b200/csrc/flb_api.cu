@@ -173,6 +173,13 @@ int grid_1d(long long n) {
   return int(b < 1 ? 1 : b);
 }
 
+// Kernels that read a block in chunks of ReadWidth cells: one chunk a thread up
+// to 8 CTAs per SM, then a grid stride (few partial results to add up).
+template <typename S>
+int read_grid(const HostBlock& b) {
+  return std::min(grid_1d(b.padded() / ReadWidth<S>::V), 148 * 8);
+}
+
 // k_halo_pull32: enough 256-thread CTAs for one batch of HALO_BATCH records
 // per thread, so that no thread starts a second, mostly idle, round.
 int halo32_grid(long long n) {
@@ -1645,8 +1652,8 @@ int flb_compute_rhou(flb_lattice* h, uint8_t key, void* stream) {
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     return for_blocks(h, [&](const HostBlock& b) {
-      k_rhou_pull<S, R><<<grid_1d(b.padded()), 256, 0, st>>>(
-          b.L, geom_of(b), static_cast<const S*>(h->pops[h->cur]), h->flags, key,
+      k_rhou_pull<S, R, ReadWidth<S>::V><<<read_grid<S>(b), 256, 0, st>>>(
+          geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->flags, key,
           static_cast<R*>(h->rho), static_cast<R*>(h->vel), h->sp);
       return FLB_OK;
     });
@@ -1663,9 +1670,9 @@ int flb_reduce_conservation(flb_lattice* h, uint8_t key, double out[4], void* st
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     return for_blocks(h, [&](const HostBlock& b) {
-      const int grid = grid_1d(b.padded());
-      k_conservation_pull<S, R><<<grid, 256, 0, st>>>(
-          b.L, geom_of(b), static_cast<const S*>(h->pops[h->cur]), h->flags, key, h->red,
+      const int grid = read_grid<S>(b);
+      k_conservation_pull<S, R, ReadWidth<S>::V><<<grid, 256, 0, st>>>(
+          geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->flags, key, h->red,
           h->sp);
       k_sum_partials<<<1, 256, 0, st>>>(h->red, grid, 4, h->acc);  // blocks in order
       return FLB_OK;
@@ -1690,8 +1697,8 @@ int flb_tolerance_u(flb_lattice* h, uint8_t key, double* max_du, void* stream) {
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     return for_blocks(h, [&](const HostBlock& b) {
-      k_tolerance_pull<S, R><<<grid_1d(b.padded()), 256, 0, st>>>(
-          b.L, geom_of(b), static_cast<const S*>(h->pops[h->cur]), h->flags, key, h->uprev,
+      k_tolerance_pull<S, R, ReadWidth<S>::V><<<read_grid<S>(b), 256, 0, st>>>(
+          geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->flags, key, h->uprev,
           acc, h->sp);
       return FLB_OK;
     });

@@ -305,20 +305,25 @@ static __global__ void __launch_bounds__(256) k_sum_partials_dd(const double* pa
   }
 }
 
+// Up to 4 values per slot, all in one pass; the order of the additions depends
+// on nslots alone.
 static __global__ void __launch_bounds__(256) k_sum_partials(const double* partials,
                                                              int nslots, int ncomp, double* acc) {
-  __shared__ double red[256];
-  for (int k = 0; k < ncomp; ++k) {
-    double s = 0;
-    for (int b = threadIdx.x; b < nslots; b += 256) s += partials[b * ncomp + k];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double v = 0;
-      for (int t = 0; t < 256; ++t) v += red[t];
-      acc[k] += v;
-    }
-    __syncthreads();
+  __shared__ double red[8][4];
+  double s[4] = {0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nslots; b += 256)
+    for (int k = 0; k < ncomp; ++k) s[k] += partials[b * ncomp + k];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double v = warp_sum(s[k]);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < ncomp) {
+    double v = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += red[w][threadIdx.x];
+    acc[threadIdx.x] += v;
   }
 }
 

@@ -1369,73 +1369,131 @@ __device__ __forceinline__ void gather_stored(const S* pops, long long dstride, 
     v[i] = gload<S, R>(pops + i * dstride + wrap_src(g, x, y, z, i), sp.shift[i], sp.inv_scale);
 }
 
-// rho and u of cell (x,y,z) (forced moments where a porosity field is given)
-template <typename S, typename R>
-__device__ __forceinline__ void cell_rho_u(const S* pops, long long dstride, const Geom& g, int x,
-                                           int y, int z, const StepParams& sp, R alpha, R& r,
-                                           R& ux, R& uy, R& uz) {
-  R f[Q];
-  if constexpr (std::is_same<S, dev32>::value) {
-    gather_stored<S, R>(pops, dstride, g, x, y, z, sp, f);
-    R delta, den;
-    dev_moments(f, sp.rho0, alpha, delta, r, den, ux, uy, uz);
-  } else {
-    gather_R<S, R>(pops, dstride, g, x, y, z, sp, f);
-    if (sp.alpha) {
-      R den;
-      forced_moments<R>(f, alpha, r, den, ux, uy, uz);
-    } else {
-      rho_u<R>(f, r, ux, uy, uz);
-    }
-  }
-}
+// ---------------------------------------------------------------------------
+// Fields, sums and the convergence check from the current populations.  Each
+// reads 19 populations a cell and little else, so they are bound by HBM; they
+// walk chunks of V cells with the step kernels' vector gather and 32-bit index
+// arithmetic.  202^3 FP32, us: fields 147 (260 with a scalar gather, its wrap
+// rule and 64-bit divisions a cell), sums 133 (350), check 173 (1090); the bytes
+// they cannot do without take 113, 96 and 157 at 6.65 TB/s.
+template <typename S>
+struct ReadWidth {
+  static constexpr int V = std::is_same<S, __half>::value ? 4 : 2;  // cells per thread
+};
 
-template <typename S, typename R>
-__global__ void k_rhou_pull(LayoutParams L, Geom g, const S* pops, const uint8_t* flags,
-                            uint8_t key, R* rho, R* vel, StepParams sp) {
-  const long long total = L.plane * L.nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
-       c += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    if (!decode_cell(L, c, x, y, z)) continue;
-    if (!(flags[g.base + c] & key)) continue;
-    R r, ux, uy, uz;
-    cell_rho_u<S, R>(pops, L.dstride, g, x, y, z, sp,
-                     sp.alpha ? static_cast<const R*>(sp.alpha)[g.base + c] : R(0), r, ux, uy,
-                     uz);
-    rho[g.base + c] = r;
-    vel[g.base + c] = ux;
-    vel[g.base + c + L.dstride] = uy;
-    vel[g.base + c + 2 * L.dstride] = uz;
-  }
-}
-
-// Mass and momentum sums of one block: CTA b writes partials[4b .. 4b+3]
-// (k_sum_partials adds them in a fixed order).
-template <typename S, typename R>
-__global__ void __launch_bounds__(256) k_conservation_pull(LayoutParams L, Geom g, const S* pops,
-                                                           const uint8_t* flags, uint8_t key,
-                                                           double* partials, StepParams sp) {
-  double s[4] = {0, 0, 0, 0};
-  const long long total = L.plane * L.nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
-       c += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    if (!decode_cell(L, c, x, y, z)) continue;
-    if (!(flags[g.base + c] & key)) continue;
-    R f[Q];
-    gather_stored<S, R>(pops, L.dstride, g, x, y, z, sp, f);
+// Cell k of a gathered chunk.
+template <typename R, int V>
+__device__ __forceinline__ void chunk_cell(const R (&vals)[Q][V], int k, R (&f)[Q]) {
 #pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      // FP16S values come converted; FP32S deviations get their shift in FP64
-      const double v = std::is_same<S, dev32>::value ? double(f[i]) + double(sp.shift[i])
-                                                     : double(f[i]);
-      s[0] += v;
-      s[1] += cx(i) * v;
-      s[2] += cy(i) * v;
-      s[3] += cz(i) * v;
-    }
+  for (int i = 0; i < Q; ++i) f[i] = vals[i][k];
+}
+
+// rho and u of a cell from its post-stream values (forced moments where a
+// porosity is given).
+template <typename S, typename R>
+__device__ __forceinline__ void cell_moments(const StepParams& sp, const R (&f)[Q], R alpha, R& r,
+                                             R& ux, R& uy, R& uz) {
+  R den;
+  if constexpr (std::is_same<S, dev32>::value) {
+    R delta;
+    dev_moments(f, sp.rho0, alpha, delta, r, den, ux, uy, uz);
+  } else if (sp.alpha) {
+    forced_moments<R>(f, alpha, r, den, ux, uy, uz);
+  } else {
+    rho_u<R>(f, r, ux, uy, uz);
   }
+}
+
+// The chunks of a block that hold a cell with the key, grid stride: body(vals,
+// hit, cell0), hit[k] telling whether cell k of the chunk has it.
+template <typename S, typename R, int V, typename F>
+__device__ __forceinline__ void for_key_chunks(const Geom& g, long long dstride, const S* pops,
+                                               const uint8_t* flags, uint8_t key,
+                                               const StepParams& sp, F&& body) {
+  const unsigned total = unsigned(g.pitch / V) * unsigned(g.ny) * unsigned(g.nz);
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < total;
+       q += gridDim.x * blockDim.x) {
+    int x0, y, z;
+    if (!chunk_coords<V>(g, q, x0, y, z)) continue;
+    const long long cell0 = g.base + (long long)y * g.pitch + (long long)z * g.plane + x0;
+    uint8_t fl[V];
+    load_flags<V>(flags + cell0, fl);
+    bool hit[V], any = false;
+#pragma unroll
+    for (int k = 0; k < V; ++k) any |= hit[k] = x0 + k < g.nx && (fl[k] & key);
+    if (!any) continue;
+    R vals[Q][V];
+    gather_chunk<S, R, V, 1>(pops, dstride, g, sp.shift, sp.inv_scale, x0, y, z, vals);
+    body(vals, hit, cell0);
+  }
+}
+
+template <typename S, typename R, int V>
+__global__ void __launch_bounds__(256, 2)
+    k_rhou_pull(Geom g, long long dstride, const S* pops, const uint8_t* flags, uint8_t key,
+                R* rho, R* vel, const __grid_constant__ StepParams sp) {
+  for_key_chunks<S, R, V>(
+      g, dstride, pops, flags, key, sp,
+      [&](const R (&vals)[Q][V], const bool (&hit)[V], long long cell0) {
+        R r[V], ux[V], uy[V], uz[V];
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          R f[Q];
+          chunk_cell<R, V>(vals, k, f);
+          cell_moments<S, R>(sp, f, sp.alpha ? static_cast<const R*>(sp.alpha)[cell0 + k] : R(0),
+                             r[k], ux[k], uy[k], uz[k]);
+          all &= hit[k];
+        }
+        if (all) {
+          vstore<R, R, V>(rho + cell0, r, 0.f, 1.f);
+          vstore<R, R, V>(vel + cell0, ux, 0.f, 1.f);
+          vstore<R, R, V>(vel + cell0 + dstride, uy, 0.f, 1.f);
+          vstore<R, R, V>(vel + cell0 + 2 * dstride, uz, 0.f, 1.f);
+        } else {
+#pragma unroll
+          for (int k = 0; k < V; ++k)
+            if (hit[k]) {
+              rho[cell0 + k] = r[k];
+              vel[cell0 + k] = ux[k];
+              vel[cell0 + k + dstride] = uy[k];
+              vel[cell0 + k + 2 * dstride] = uz[k];
+            }
+        }
+      });
+}
+
+// Mass and momentum sums of one block in FP64: CTA b writes partials[4b .. 4b+3]
+// (k_sum_partials adds them in a fixed order).  Opposite populations are added
+// and subtracted in FP64 first: 47 FP64 operations a cell instead of 76.
+template <typename S, typename R, int V>
+__global__ void __launch_bounds__(256, 2)
+    k_conservation_pull(Geom g, long long dstride, const S* pops, const uint8_t* flags,
+                        uint8_t key, double* partials, const __grid_constant__ StepParams sp) {
+  double s[4] = {0, 0, 0, 0};
+  for_key_chunks<S, R, V>(
+      g, dstride, pops, flags, key, sp,
+      [&](const R (&vals)[Q][V], const bool (&hit)[V], long long) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          if (!hit[k]) continue;
+          // FP16S values come converted; FP32S deviations get their shift in FP64
+          auto value = [&](int i) {
+            return std::is_same<S, dev32>::value ? double(vals[i][k]) + double(sp.shift[i])
+                                                 : double(vals[i][k]);
+          };
+          double m = value(0);
+#pragma unroll
+          for (int i = 1; i < Q; i += 2) {
+            const double a = value(i), b = value(i + 1), d = a - b;
+            m += a + b;
+            if (cx(i)) s[1] += cx(i) > 0 ? d : -d;
+            if (cy(i)) s[2] += cy(i) > 0 ? d : -d;
+            if (cz(i)) s[3] += cz(i) > 0 ? d : -d;
+          }
+          s[0] += m;
+        }
+      });
   __shared__ double red[8][4];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
@@ -1451,36 +1509,63 @@ __global__ void __launch_bounds__(256) k_conservation_pull(LayoutParams L, Geom 
   }
 }
 
-template <typename S, typename R>
-__global__ void __launch_bounds__(256) k_tolerance_pull(LayoutParams L, Geom g, const S* pops,
-                                                        const uint8_t* flags, uint8_t key,
-                                                        double* uprev, unsigned long long* acc,
-                                                        StepParams sp) {
+template <typename S, typename R, int V>
+__global__ void __launch_bounds__(256, 2)
+    k_tolerance_pull(Geom g, long long dstride, const S* pops, const uint8_t* flags, uint8_t key,
+                     double* uprev, unsigned long long* acc,
+                     const __grid_constant__ StepParams sp) {
   double m = 0;
-  const long long total = L.plane * L.nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
-       c += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    if (!decode_cell(L, c, x, y, z)) continue;
-    if (!(flags[g.base + c] & key)) continue;
-    R r, ux, uy, uz;
-    if constexpr (std::is_same<S, dev32>::value) {
-      cell_rho_u<S, R>(pops, L.dstride, g, x, y, z, sp, R(0), r, ux, uy, uz);
-    } else {
-      R f[Q];
-      gather_R<S, R>(pops, L.dstride, g, x, y, z, sp, f);
-      rho_u<R>(f, r, ux, uy, uz);
-    }
-    const double u[3] = {double(ux), double(uy), double(uz)};
+  for_key_chunks<S, R, V>(
+      g, dstride, pops, flags, key, sp,
+      [&](const R (&vals)[Q][V], const bool (&hit)[V], long long cell0) {
+        // the old velocities first, all at once: each read after the store of
+        // the one before, they are six trips to memory in a row
+        double old[3][V];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      double* up = uprev + g.base + c + d * L.dstride;
-      m = fmax(m, fabs(u[d] - *up));
-      *up = u[d];
-    }
-  }
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int k = 0; k < V; k += 2) {
+            const double2 w = *reinterpret_cast<const double2*>(uprev + cell0 + d * dstride + k);
+            old[d][k] = w.x;
+            old[d][k + 1] = w.y;
+          }
+        double u[3][V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+          R f[Q], r, ux, uy, uz;
+          chunk_cell<R, V>(vals, k, f);
+          if constexpr (std::is_same<S, dev32>::value) {
+            R delta, den;
+            dev_moments(f, sp.rho0, R(0), delta, r, den, ux, uy, uz);
+          } else {
+            rho_u<R>(f, r, ux, uy, uz);
+          }
+          u[0][k] = ux;
+          u[1][k] = uy;
+          u[2][k] = uz;
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int k = 0; k < V; ++k) {
+            if (hit[k]) m = fmax(m, fabs(u[d][k] - old[d][k]));
+            else u[d][k] = old[d][k];
+          }
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int k = 0; k < V; k += 2)
+            *reinterpret_cast<double2*>(uprev + cell0 + d * dstride + k) =
+                make_double2(u[d][k], u[d][k + 1]);
+      });
+  __shared__ double red[8];
   m = warp_max(m);
-  if ((threadIdx.x & 31) == 0) atomicMax(acc, (unsigned long long)__double_as_longlong(m));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, red[w]);
+    atomicMax(acc, (unsigned long long)__double_as_longlong(m));
+  }
 }
 
 // Halo in pull form: the overlap value R_b(g, i) lives in P_b at
