@@ -122,6 +122,7 @@ struct flb_lattice {
   double wait_s = 2.0;     // bound of one device-side wait (k_pull_tma)
   long long withhold = -1; // failure-detection test hook (flb_test_withhold_tile)
   int vec = 0;  // cells per thread of the step kernel; 0 = storage default
+  bool shape_chosen = false;  // by flb_set_launch or flb_autotune; else auto_shape
   int rounding = FLB_ROUND_DEFAULT;  // FP16S stores (flb_set_rounding)
   alignas(8) char snap_hdr[64] = {};  // source of the snapshot header copies
   // CUDA graphs of the two-step cycle, one per starting buffer parity
@@ -293,6 +294,51 @@ int default_vec(int storage) { return storage == FLB_STORAGE_FP16S ? 4 : 2; }
 int vec_width(const flb_lattice* h) { return h->vec ? h->vec : default_vec(h->desc.storage); }
 bool vec_allowed(int storage, int v) {
   return storage == FLB_STORAGE_FP64 ? (v == 1 || v == 2) : (v == 2 || v == 4);
+}
+bool tma_supported(const flb_lattice* h);
+
+// Launch shape of one step.
+struct Shape {
+  int tile_y, ctas_per_sm, vec;
+};
+
+// Shape of a handle's steps until flb_set_launch or flb_autotune chooses one.
+// Measured on cavities (us a step at 32 / 64 / 96 / 128 / 192 / 256 / 320 stored
+// cells a side):
+//   FP16S BGK  2 cells a thread   6.2 / 10.3 / 20.5 / 52 / 153 / 349 / 653
+//              4 cells a thread  10.3 / 11.3 / 20.5 / 46 / 128 / 285 / 538
+//              bulk copy (-2)    10.3 / 14.4 / 24.6 / 43 / 114 / 262 / 479
+//   FP16S MRT  2 cells a thread   6.2 / 11.3 / 22.6 / 55 / 159 / 366 / 682
+//              4 cells a thread  10.5 / 12.3 / 25.4 / 57 / 166 / 339 / 665
+//              bulk copy (-2)    10.3 / 14.4 / 27.3 / 49 / 130 / 307 / 547
+//   FP16S LES  2 cells a thread   6.2 / 10.5 / 22.4 / 54 / 158 / 364 / 682
+//              4 cells a thread  10.3 / 12.3 / 24.0 / 51 / 149 / 325 / 600
+//              bulk copy (-2)    10.3 / 14.4 / 26.7 / 48 / 128 / 296 / 534
+// Small lattices are bound by one thread's chain of work, so fewer cells a
+// thread; large FP16S ones by the loads in flight, which the bulk copies take
+// off the registers.  The line between them lies at 1.2 M cells (106^3): the
+// sides meet between 96^3 and 128^3.  Where the rows do not suit the bulk
+// copies, BGK and LES change to 4 cells a thread there and MRT (whose 4-cell
+// form spills) at 10 M cells (between 192^3 and 256^3).
+// Many blocks (4 warps each; one tile a CTA / persistent, 32 CTAs an SM): FP32
+// at 2 / 4 cells a thread, 48 uneven blocks of 256^3 739 / 622 us, 16 cavities of
+// 32 to 128 388 / 347 us, 160^3 in blocks with LES 180 / 163 us; FP16S at 4 cells
+// 431 / 417, 262 / 259 and (MRT) 125 / 122 us; FP64 at 2 cells 1242 / 1224 us.
+// FP32S keeps one tile a CTA at 2 cells.  FP64 keeps 2 cells a thread: 1 cell and 2
+// warps took 102 / 770 us instead of 111 / 810 at 128^3 / 256^3, but 148 instead of
+// 140 us on a 143 x 162 x 120 box.
+Shape auto_shape(const flb_lattice* h) {
+  const int storage = h->desc.storage;
+  if (h->mode >= 0) {
+    if (storage == FLB_STORAGE_FP32S) return {4, 0, 2};
+    return {4, 32, storage == FLB_STORAGE_FP64 ? 2 : 4};
+  }
+  const HostBlock& b = h->blocks[0];
+  const long long cells = (long long)b.L.nx * b.L.ny * b.L.nz;
+  const bool large = cells >= 1200000;
+  if (storage != FLB_STORAGE_FP16S) return {4, 0, 2};
+  if (large && tma_supported(h)) return {4, -2, 4};
+  return {4, 0, (h->desc.model == FLB_MODEL_MRT ? cells >= 10000000 : large) ? 4 : 2};
 }
 
 Geom geom_of(const HostBlock& b) {
@@ -864,6 +910,17 @@ int flags_any(flb_lattice* h, int b, uint8_t* host, bool upload, void* stream) {
   return FLB_OK;
 }
 
+// Give a handle without a chosen shape its default one.
+int apply_auto_shape(flb_lattice* h) {
+  if (h->shape_chosen) return FLB_OK;
+  const Shape s = auto_shape(h);
+  if (s.ctas_per_sm <= -2) FLB_TRY(tma_prepare(h));
+  h->tile_y = s.tile_y;
+  h->ctas_per_sm = s.ctas_per_sm;
+  h->vec = s.vec;
+  return FLB_OK;
+}
+
 // Common allocation for flb_create / flb_create_blocks.
 int create_common(const flb_lattice_desc* desc, std::vector<HostBlock> blocks, int mode,
                   flb_lattice** out) {
@@ -914,6 +971,7 @@ int create_common(const flb_lattice_desc* desc, std::vector<HostBlock> blocks, i
       return cleanup(fail(FLB_ERR_OOM, "cudaMalloc alpha: %s", cudaGetErrorString(e)));
   }
   build_params(h);
+  if (int rc0 = apply_auto_shape(h)) return cleanup(rc0);
   if (int rc0 = upload_op_lut(h)) return cleanup(rc0);
   for (const HostBlock& b : h->blocks)
     if ((long long)(b.L.pitch) * b.L.ny * b.L.nz >= (1LL << 32))
@@ -1059,6 +1117,7 @@ int flb_set_tasks(flb_lattice* h, int ntasks, const uint8_t* keys, const uint8_t
   h->sp.src = keep.src;
   h->sp.dst = keep.dst;
   drop_graphs(h);
+  FLB_TRY(apply_auto_shape(h));
   return upload_op_lut(h);
 }
 
@@ -1488,6 +1547,7 @@ int flb_set_launch(flb_lattice* h, int tile_y, int ctas_per_sm, int cells_per_th
   h->tile_y = tile_y;
   h->ctas_per_sm = ctas_per_sm;
   h->vec = v;
+  h->shape_chosen = true;
   return FLB_OK;
 }
 

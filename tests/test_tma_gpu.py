@@ -144,3 +144,23 @@ def test_tma_wait_that_gives_up_is_reported_and_the_handle_recovers(gpu_ok):
     lat.step(steps)
     lat.device_status()
     assert np.array_equal(lat.download_pops(), ref.download_pops())
+
+
+@pytest.mark.parametrize("ni,model,want", [
+    (104, "bgk", (4, 0, 2)),    # 106^3: the last size below the line
+    (106, "bgk", (4, 0, 4)),    # 108^3: above it, rows not on 16-byte boundaries
+    (106, "mrt", (4, 0, 2)),
+    (108, "bgk", (4, -2, 4)),   # 110^3: rows of 112
+    (110, "les", (4, -2, 4)),
+    (110, "mrt", (4, -2, 4)),
+])
+def test_default_shape_gives_the_direct_kernels_bits(gpu_ok, ni, model, want):
+    """The shape the library picks by itself, on both sides of each line of its
+    rule, and the one it picks again when the model changes."""
+    a, b = (F.cavity(ni, tau=0.55, storage="fp16s", model=model) for _ in range(2))
+    assert a.get_launch() == want
+    b.set_launch(1, 0, 4)
+    a.step(6)
+    b.step(6)
+    a.device_status()
+    assert np.array_equal(a.download_pops(), b.download_pops())
