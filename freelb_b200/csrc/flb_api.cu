@@ -629,6 +629,14 @@ StepParams block_half_params(const flb_lattice* h) {
   return p;
 }
 
+// Lattices that k_pull steps in its SMALL form: up to 300,000 padded cells, 64^3
+// and the like.  Us a step in a graph of two, without / with it, at 32 / 48 / 64 /
+// 72 stored cells a side: FP32 BGK 5.13 / 7.16 / 9.42 / 12.2 and 4.12 / 6.16 /
+// 9.25 / 12.3, LES 4.38 / 7.19 / 10.3 / 12.8 and 5.13 / 6.16 / 10.3 / 13.3 (12^3:
+// 5.14 and 4.13), FP16S BGK 6.16 / 6.34 / 9.71 / 11.3 and 4.12 / 5.15 / 7.21 / 9.61,
+// FP64 5.15 / 8.21 / 15.4 / 23.7 and 5.16 / 7.20 / 15.4 / 23.6.
+bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
+
 template <typename S, typename R, int MODEL, int V>
 void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
   if constexpr (std::is_same<S, __half>::value && V == 4 && MODEL != MODEL_BRINKMAN) {
@@ -674,6 +682,16 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
     const long long chunks = (long long)(b.L.pitch / V) * b.L.ny * b.L.nz;
     const long long per_cta = 32LL * h->tile_y;
     const dim3 grid(unsigned((chunks + per_cta - 1) / per_cta));
+    if constexpr (V == 2) {
+      if (small_lattice(b)) {
+        if constexpr (std::is_same<S, __half>::value)
+          k_pull<S, R, MODEL, V, true><<<grid, dim3(32 * h->tile_y), 0, st>>>(
+              half_step_params<V>(h));
+        else
+          k_pull<S, R, MODEL, V, true><<<grid, dim3(32 * h->tile_y), 0, st>>>(h->sp);
+        return;
+      }
+    }
     if constexpr (std::is_same<S, __half>::value && V >= 2)
       k_pull<S, R, MODEL, V><<<grid, dim3(32 * h->tile_y), 0, st>>>(half_step_params<V>(h));
     else

@@ -118,6 +118,17 @@ __device__ __forceinline__ long long wrap_off(const Geom& g, int x, int y, int z
   return g.base + sx + (long long)sy * g.pitch + (long long)sz * g.plane;
 }
 
+// The same cell from its linear row r0 = z * ny + y (see below): one carry for x,
+// one wrap of the row, no test of y or z.
+__device__ __forceinline__ long long wrap_row_off(const Geom& g, int x, int r0, int dx, int dr) {
+  int sx = x + dx, r = r0 + dr;
+  if (dx < 0 && sx < 0) { sx += g.nx; --r; }
+  if (dx > 0 && sx >= g.nx) { sx -= g.nx; ++r; }
+  const int rows = g.ny * g.nz;
+  r = r < 0 ? r + rows : r >= rows ? r - rows : r;
+  return g.base + (long long)r * g.pitch + sx;
+}
+
 // Linear rows.  Rows are numbered r = z * ny + y over the block and the padded
 // layout stores row r at r * pitch, so the carry of y into z in the reference's
 // periodic shift over the linear cell index (CyclicArray::rotate,
@@ -145,7 +156,11 @@ __device__ __forceinline__ bool interior_row(const Geom& g, int y, int z) {
 // row end then re-load through the wrap rule; the rows near the block's first
 // and last planes (not interior) take every source through it.  Called for
 // chunks with x0 < nx only.
-template <typename S, typename R, int V, int SIGN>
+//
+// ROWS: the wrap rule on linear rows (wrap_row_off), straight-line code whose
+// loads are all in flight together; the cell-wise rule branches from load to
+// load, but needs fewer registers.
+template <typename S, typename R, int V, int SIGN, bool ROWS = false>
 __device__ __forceinline__ void gather_chunk(const S* __restrict__ arr, long long dstride,
                                              const Geom& g, const float* shift, float inv_scale,
                                              int x0, int y, int z, R (&vals)[Q][V]) {
@@ -208,10 +223,13 @@ __device__ __forceinline__ void gather_chunk(const S* __restrict__ arr, long lon
     for (int k = 0; k < V; ++k) {
       const int x = min(x0 + k, g.nx - 1);
 #pragma unroll
-      for (int i = 0; i < Q; ++i)
-        vals[i][k] = gload<S, R>(
-            arr + i * dstride + wrap_off(g, x, y, z, -SIGN * cx(i), -SIGN * cy(i), -SIGN * cz(i)),
-            shift[i], inv_scale);
+      for (int i = 0; i < Q; ++i) {
+        const long long at =
+            ROWS ? wrap_row_off(g, x, z * g.ny + y, -SIGN * cx(i),
+                                -SIGN * (cy(i) + g.ny * cz(i)))
+                 : wrap_off(g, x, y, z, -SIGN * cx(i), -SIGN * cy(i), -SIGN * cz(i));
+        vals[i][k] = gload<S, R>(arr + i * dstride + at, shift[i], inv_scale);
+      }
     }
   }
 }
@@ -320,7 +338,7 @@ __device__ __forceinline__ uint2 hsplice_next(uint2 v, uint2 w) {
 // components per D3Q19 velocity the carry reaches z only when the y row wraps,
 // and then c_z = 0.
 // Rows near the block's first and last planes: every source through the wrap rule.
-template <int V>
+template <int V, bool ROWS = false>
 __device__ __forceinline__ void gather_words_wrap(const __half* __restrict__ arr,
                                                   long long dstride, const Geom& g, int x0,
                                                   int y, int z, typename HWord<V>::type (&h)[Q]) {
@@ -332,7 +350,10 @@ __device__ __forceinline__ void gather_words_wrap(const __half* __restrict__ arr
     const int x = min(x0 + k, g.nx - 1);
 #pragma unroll
     for (int i = 0; i < Q; ++i)
-      hset(h[i], k, hscalar(arr + i * dstride + wrap_off(g, x, y, z, -cx(i), -cy(i), -cz(i))));
+      hset(h[i], k,
+           hscalar(arr + i * dstride +
+                   (ROWS ? wrap_row_off(g, x, z * g.ny + y, -cx(i), -(cy(i) + g.ny * cz(i)))
+                         : wrap_off(g, x, y, z, -cx(i), -cy(i), -cz(i)))));
   }
 }
 
@@ -1100,7 +1121,7 @@ __device__ __forceinline__ void pull_chunk_half(const StepParams& p, const Geom&
 
 // Single-block FP16S chunk (19 * dstride < 2^32): linear row `row`, first cell
 // `cell` = row * pitch + x0; sources and stores through the direction bases.
-template <int MODEL, int V>
+template <int MODEL, int V, bool ROWS = false>
 __device__ __forceinline__ void pull_chunk_half32(const StepParams& p, const Geom& g, float omega,
                                                   int x0, unsigned row, unsigned cell) {
   typename HWord<V>::type h[Q];
@@ -1108,8 +1129,8 @@ __device__ __forceinline__ void pull_chunk_half32(const StepParams& p, const Geo
     gather_words_dir<V>(p, g, x0, cell, h);
   } else {
     const unsigned z = row / unsigned(g.ny);
-    gather_words_wrap<V>(static_cast<const __half*>(p.src), p.dstride, g, x0,
-                         int(row - z * unsigned(g.ny)), int(z), h);
+    gather_words_wrap<V, ROWS>(static_cast<const __half*>(p.src), p.dstride, g, x0,
+                               int(row - z * unsigned(g.ny)), int(z), h);
   }
   uint8_t fl[V];
   load_flags<V>(p.flags + cell, fl);
@@ -1188,7 +1209,7 @@ __device__ __forceinline__ void pull_chunk_half_blk32(const StepParams& p, const
   for (int i = 0; i < Q; ++i) hstore<V>(static_cast<__half*>(p.dst_dir[i]) + cell, h[i]);
 }
 
-template <typename S, typename R, int MODEL, int V>
+template <typename S, typename R, int MODEL, int V, bool ROWS = false>
 __device__ __forceinline__ void pull_chunk(const StepParams& p, const Geom& g, R omega, int lane,
                                            int x0, int y, int z) {
   if constexpr (std::is_same<S, __half>::value && V >= 2) {
@@ -1198,7 +1219,7 @@ __device__ __forceinline__ void pull_chunk(const StepParams& p, const Geom& g, R
   const S* __restrict__ src = static_cast<const S*>(p.src);
   S* __restrict__ dst = static_cast<S*>(p.dst);
   R vals[Q][V];
-  gather_chunk<S, R, V, 1>(src, p.dstride, g, p.shift, p.inv_scale, x0, y, z, vals);
+  gather_chunk<S, R, V, 1, ROWS>(src, p.dstride, g, p.shift, p.inv_scale, x0, y, z, vals);
   const int nvalid = min(V, g.nx - x0);
   const long long cell0 = g.base + (long long)y * g.pitch + (long long)z * g.plane + x0;
   uint8_t fl[V];
@@ -1263,8 +1284,15 @@ struct PullBounds {
                                                               : 3;
 };
 
-template <typename S, typename R, int MODEL, int V>
-__global__ void __launch_bounds__(256, PullBounds<S, MODEL, V>::min_ctas) k_pull(const StepParams p) {
+//
+// SMALL: lattices that do not fill the GPU (small_lattice in flb_api.cu), where
+// a step takes as long as one thread's chain of work.  The longest chain is that
+// of the rows near the first and last planes, so it takes the straight-line wrap
+// rule, and the registers that needs, which would cost a full GPU its warps
+// (100^3 FP32: 31.1 us a step as it is, 34.9 in this form).
+template <typename S, typename R, int MODEL, int V, bool SMALL = false>
+__global__ void __launch_bounds__(256, SMALL ? 1 : PullBounds<S, MODEL, V>::min_ctas)
+    k_pull(const StepParams p) {
   const Geom g{p.nx, p.ny, p.nz, p.pitch, p.plane, 0};
   if constexpr (std::is_same<S, __half>::value && V >= 2) {
     // 32-bit chunk index (fewer than 2^31 chunks: 19 * dstride < 2^32)
@@ -1274,13 +1302,13 @@ __global__ void __launch_bounds__(256, PullBounds<S, MODEL, V>::min_ctas) k_pull
     const unsigned row = p.cpr_m ? __umulhi(q, p.cpr_m) >> (p.cpr_s - 1) : q;
     const int x0 = int(q - row * cpr) * V;
     if (x0 >= p.nx) return;
-    pull_chunk_half32<MODEL, V>(p, g, float(p.omega), x0, row, q * V);
+    pull_chunk_half32<MODEL, V, SMALL>(p, g, float(p.omega), x0, row, q * V);
     return;
   }
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int x0, y, z;
   if (!chunk_coords<V>(g, q, x0, y, z)) return;
-  pull_chunk<S, R, MODEL, V>(p, g, R(p.omega), 0, x0, y, z);
+  pull_chunk<S, R, MODEL, V, SMALL>(p, g, R(p.omega), 0, x0, y, z);
 }
 
 // Many blocks: tiles of blockDim.x consecutive chunks, numbered block by block

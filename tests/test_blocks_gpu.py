@@ -234,3 +234,28 @@ def test_full_halo_matches_oracle(gpu_ok, storage, tol):
     assert rel_maxnorm(pops, want) < tol
     lat.set_halo_mode("normal")
     assert lat.halo_count() == normal
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s", "fp64", "fp32s"])
+@pytest.mark.parametrize("dims", [(3, 3, 3), (5, 9, 4), (100, 60, 50), (100, 60, 51)])
+def test_small_lattice_form_equals_the_tile_kernel(gpu_ok, storage, dims):
+    """The step kernel's form for small lattices (up to 300,000 padded cells: the
+    third shape is the last of them) against the tile kernel, bit for bit, on
+    every row near the first and last planes and with every op."""
+    n = dims[0] * dims[1] * dims[2]
+    rng = np.random.default_rng(n)
+    flags = rng.choice(np.array([1, 2, 4, 8, 16], dtype=np.uint8), size=n, p=[.1, .6, .1, .1, .1])
+    tasks = ((2, "bulk"), (4, "bounceback"), (8, "movingwall"), (16, "field_bgk"))
+    pops = np.repeat(O.W, n) * (1 + 0.05 * rng.standard_normal(19 * n))
+    u = 0.03 * rng.standard_normal(3 * n)
+    out = []
+    for shape in ((4, 0, 2), (8, 16, 2)):
+        lat = F.Lattice(*dims, 0.57, storage=storage, tasks=tasks)
+        lat.upload_flags(flags)
+        lat.upload_pops(pops)
+        lat.upload_field("u", u)
+        lat.set_launch(*shape)
+        lat.step(5)
+        out.append(lat.download_pops())
+        lat.close()
+    assert np.array_equal(out[0], out[1])
