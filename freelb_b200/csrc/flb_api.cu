@@ -102,6 +102,7 @@ struct flb_lattice {
   double* uprev = nullptr;
   uint8_t* d_lut = nullptr;  // op of every flag value
   StepParams sp{};
+  bool dependent = false;  // the step's launches carry the dependent-launch attribute
   // multi-block launch data
   BlockEntry* d_blocks = nullptr;
   int* d_tile_block = nullptr;  // block of every tile (tile kernel)
@@ -668,9 +669,11 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
       const long long ctas_needed = ((chunks + 31) / 32 + PIPE_WARPS - 1) / PIPE_WARPS;
       const long long g = std::max(1LL, std::min(ctas_needed, (long long)h->pipe_ctas * h->sm_count));
       if (pipe_wide(h))
-        k_pull_pipe<MODEL, true><<<unsigned(g), PIPE_WARPS * 32, pipe_smem_bytes(), st>>>(h->sp);
+        launch_dependent(h->dependent, k_pull_pipe<MODEL, true>, unsigned(g), PIPE_WARPS * 32,
+                         pipe_smem_bytes(), st, h->sp);
       else
-        k_pull_pipe<MODEL, false><<<unsigned(g), PIPE_WARPS * 32, pipe_smem_bytes(), st>>>(h->sp);
+        launch_dependent(h->dependent, k_pull_pipe<MODEL, false>, unsigned(g), PIPE_WARPS * 32,
+                         pipe_smem_bytes(), st, h->sp);
       return;
     }
   }
@@ -685,29 +688,33 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
     if constexpr (V == 2) {
       if (small_lattice(b)) {
         if constexpr (std::is_same<S, __half>::value)
-          k_pull<S, R, MODEL, V, true><<<grid, dim3(32 * h->tile_y), 0, st>>>(
-              half_step_params<V>(h));
+          launch_dependent(h->dependent, k_pull<S, R, MODEL, V, true>, grid,
+                           dim3(32 * h->tile_y), 0, st, half_step_params<V>(h));
         else
-          k_pull<S, R, MODEL, V, true><<<grid, dim3(32 * h->tile_y), 0, st>>>(h->sp);
+          launch_dependent(h->dependent, k_pull<S, R, MODEL, V, true>, grid,
+                           dim3(32 * h->tile_y), 0, st, h->sp);
         return;
       }
     }
     if constexpr (std::is_same<S, __half>::value && V >= 2)
-      k_pull<S, R, MODEL, V><<<grid, dim3(32 * h->tile_y), 0, st>>>(half_step_params<V>(h));
+      launch_dependent(h->dependent, k_pull<S, R, MODEL, V>, grid,
+                       dim3(32 * h->tile_y), 0, st, half_step_params<V>(h));
     else
-      k_pull<S, R, MODEL, V><<<grid, dim3(32 * h->tile_y), 0, st>>>(h->sp);
+      launch_dependent(h->dependent, k_pull<S, R, MODEL, V>, grid,
+                       dim3(32 * h->tile_y), 0, st, h->sp);
   } else {
     long long g = h->ctas_per_sm > 0 ? (long long)h->ctas_per_sm * h->sm_count : h->ntiles;
     g = std::max(1LL, std::min(g, h->ntiles));
     if constexpr (std::is_same<S, __half>::value && V >= 2) {
       if ((long long)Q * h->dstride < (1LL << 32)) {
-        k_pull_blocks_half32<MODEL, V><<<unsigned(g), dim3(32 * h->tile_y), 0, st>>>(
-            block_half_params(h), h->d_blocks, h->d_tile_block, h->ntiles);
+        launch_dependent(h->dependent, k_pull_blocks_half32<MODEL, V>, unsigned(g),
+                         dim3(32 * h->tile_y), 0, st, block_half_params(h), h->d_blocks,
+                         h->d_tile_block, h->ntiles);
         return;
       }
     }
-    k_pull_blocks<S, R, MODEL, V><<<unsigned(g), dim3(32 * h->tile_y), 0, st>>>(
-        h->sp, h->d_blocks, h->d_tile_block, h->ntiles);
+    launch_dependent(h->dependent, k_pull_blocks<S, R, MODEL, V>, unsigned(g),
+                     dim3(32 * h->tile_y), 0, st, h->sp, h->d_blocks, h->d_tile_block, h->ntiles);
   }
 }
 
@@ -723,8 +730,9 @@ void launch_one_step(flb_lattice* h, cudaStream_t st) {
   }
   if (h->nhalo > 0) {
     if (h->halo32)
-      k_halo_pull32<S><<<halo32_grid(h->nhalo), 256, 0, st>>>(
-          reinterpret_cast<const uint2*>(h->d_halo), h->nhalo, static_cast<S*>(h->sp.dst));
+      launch_dependent(h->dependent, k_halo_pull32<S>, halo32_grid(h->nhalo), 256, 0, st,
+                       reinterpret_cast<const uint2*>(h->d_halo), h->nhalo,
+                       static_cast<S*>(h->sp.dst));
     else
       k_halo_pull<S><<<grid_1d(h->nhalo), 256, 0, st>>>(h->d_halo, h->nhalo,
                                                         static_cast<S*>(h->sp.dst), h->dstride);
@@ -734,6 +742,7 @@ void launch_one_step(flb_lattice* h, cudaStream_t st) {
 template <typename S, typename R>
 int launch_steps(flb_lattice* h, int nsteps, cudaStream_t st) {
   if (h->mode >= 0 || h->ctas_per_sm > 0) FLB_TRY(upload_block_table(h));
+  h->dependent = may_depend(st);
   for (int s = 0; s < nsteps; ++s) {
     h->sp.src = h->pops[h->cur];
     h->sp.dst = h->pops[h->cur ^ 1];
@@ -767,6 +776,7 @@ int step_between(flb_lattice* h, const void* src, void* dst, cudaStream_t st) {
   void* d0 = h->sp.dst;
   h->sp.src = src;
   h->sp.dst = dst;
+  h->dependent = may_depend(st);
   int rc = with_types(h, [&](auto* sp, auto* rp) {
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;

@@ -78,8 +78,10 @@ __device__ __forceinline__ R dot_c(R ux, R uy, R uz, int j) {
 // and the links in cell order.
 template <typename S, typename R, int KIND>
 __global__ void __launch_bounds__(256) k_bb(const BBArgs a, S* pops) {
+  start_dependents();
   const R* rho = static_cast<const R*>(a.rho);
   const R* vel = static_cast<const R*>(a.vel);
+  wait_prerequisites();
   for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < a.n;
        r += (long long)gridDim.x * blockDim.x) {
     const uint2 link = __ldg(a.link + r);
@@ -143,17 +145,20 @@ int launch(flb_bb* bb, flb_lattice* lat, cudaStream_t st) {
   if (blocks > 148 * 32) blocks = 148 * 32;
   if (blocks < 1) blocks = 1;
   S* p = static_cast<S*>(pops);
+  auto go = [&](void (*kernel)(BBArgs, S*)) {
+    launch_dependent(may_depend(st), kernel, unsigned(blocks), 256, 0, st, a, p);
+  };
   switch (bb->kind) {
-    case FLB_BB_NORMAL: k_bb<S, R, FLB_BB_NORMAL><<<unsigned(blocks), 256, 0, st>>>(a, p); break;
+    case FLB_BB_NORMAL: go(k_bb<S, R, FLB_BB_NORMAL>); break;
     case FLB_BB_MOVINGWALL:
-      k_bb<S, R, FLB_BB_MOVINGWALL><<<unsigned(blocks), 256, 0, st>>>(a, p);
+      go(k_bb<S, R, FLB_BB_MOVINGWALL>);
       break;
     case FLB_BB_ANTI_SIMPLE:
-      k_bb<S, R, FLB_BB_ANTI_SIMPLE><<<unsigned(blocks), 256, 0, st>>>(a, p);
+      go(k_bb<S, R, FLB_BB_ANTI_SIMPLE>);
       break;
-    case FLB_BB_ANTI_O1: k_bb<S, R, FLB_BB_ANTI_O1><<<unsigned(blocks), 256, 0, st>>>(a, p); break;
-    case FLB_BB_ANTI_O2: k_bb<S, R, FLB_BB_ANTI_O2><<<unsigned(blocks), 256, 0, st>>>(a, p); break;
-    default: k_bb<S, R, FLB_BB_ANTI_PRESSURE><<<unsigned(blocks), 256, 0, st>>>(a, p); break;
+    case FLB_BB_ANTI_O1: go(k_bb<S, R, FLB_BB_ANTI_O1>); break;
+    case FLB_BB_ANTI_O2: go(k_bb<S, R, FLB_BB_ANTI_O2>); break;
+    default: go(k_bb<S, R, FLB_BB_ANTI_PRESSURE>); break;
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

@@ -205,6 +205,8 @@ __device__ __forceinline__ void pipe_compute(const StepParams& p, const Geom& g,
 template <int MODEL, bool WIDE>
 __global__ void __launch_bounds__(PIPE_WARPS * 32, FLB_PIPE_MIN_CTAS)
     k_pull_pipe(const StepParams p) {
+  start_dependents();
+  wait_prerequisites();
   extern __shared__ __align__(16) unsigned char pipe_smem[];
   const int lane = int(threadIdx.x) & 31, warp = int(threadIdx.x) >> 5;
   PipeStage* st = reinterpret_cast<PipeStage*>(pipe_smem) + 2 * warp;

@@ -1293,6 +1293,7 @@ struct PullBounds {
 template <typename S, typename R, int MODEL, int V, bool SMALL = false>
 __global__ void __launch_bounds__(256, SMALL ? 1 : PullBounds<S, MODEL, V>::min_ctas)
     k_pull(const StepParams p) {
+  start_dependents();
   const Geom g{p.nx, p.ny, p.nz, p.pitch, p.plane, 0};
   if constexpr (std::is_same<S, __half>::value && V >= 2) {
     // 32-bit chunk index (fewer than 2^31 chunks: 19 * dstride < 2^32)
@@ -1302,12 +1303,14 @@ __global__ void __launch_bounds__(256, SMALL ? 1 : PullBounds<S, MODEL, V>::min_
     const unsigned row = p.cpr_m ? __umulhi(q, p.cpr_m) >> (p.cpr_s - 1) : q;
     const int x0 = int(q - row * cpr) * V;
     if (x0 >= p.nx) return;
+    wait_prerequisites();
     pull_chunk_half32<MODEL, V, SMALL>(p, g, float(p.omega), x0, row, q * V);
     return;
   }
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int x0, y, z;
   if (!chunk_coords<V>(g, q, x0, y, z)) return;
+  wait_prerequisites();
   pull_chunk<S, R, MODEL, V, SMALL>(p, g, R(p.omega), 0, x0, y, z);
 }
 
@@ -1318,6 +1321,8 @@ template <typename S, typename R, int MODEL, int V>
 __global__ void __launch_bounds__(256, PullBounds<S, MODEL, V>::min_ctas)
     k_pull_blocks(const StepParams p, const BlockEntry* __restrict__ blocks,
                   const int* __restrict__ tile_block, long long ntiles) {
+  start_dependents();
+  wait_prerequisites();
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BlockEntry& b = blocks[__ldg(tile_block + t)];
     const long long q = (t - b.tile_start) * blockDim.x + threadIdx.x;
@@ -1332,6 +1337,8 @@ template <int MODEL, int V>
 __global__ void __launch_bounds__(256, PullBounds<__half, MODEL, V>::min_ctas)
     k_pull_blocks_half32(const StepParams p, const BlockEntry* __restrict__ blocks,
                          const int* __restrict__ tile_block, long long ntiles) {
+  start_dependents();
+  wait_prerequisites();
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BlockEntry& b = blocks[__ldg(tile_block + t)];
     const long long q = (t - b.tile_start) * blockDim.x + threadIdx.x;
@@ -1625,6 +1632,8 @@ constexpr int HALO_BATCH = 4;
 
 template <typename S>
 __global__ void k_halo_pull32(const uint2* __restrict__ recs, long long n, S* pops) {
+  start_dependents();
+  wait_prerequisites();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long r0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; r0 < n;
        r0 += stride * HALO_BATCH) {
