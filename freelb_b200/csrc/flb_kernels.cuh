@@ -326,7 +326,7 @@ __device__ __forceinline__ dd warp_sum_dd(dd v) {
 // += the rounded double-double total (k_objective).
 static __global__ void __launch_bounds__(256) k_sum_partials_dd(const double* partials,
                                                                 int nslots, double* acc) {
-  __shared__ double red[2][256];
+  __shared__ double red[2][8];
   dd s;
   for (int b = threadIdx.x; b < nslots; b += 256) {
     dd v;
@@ -334,12 +334,15 @@ static __global__ void __launch_bounds__(256) k_sum_partials_dd(const double* pa
     v.lo = partials[2 * b + 1];
     s.add(v);
   }
-  red[0][threadIdx.x] = s.hi;
-  red[1][threadIdx.x] = s.lo;
+  s = warp_sum_dd(s);
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = s.hi;
+    red[1][threadIdx.x >> 5] = s.lo;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     dd t;
-    for (int k = 0; k < 256; ++k) {
+    for (int k = 0; k < 8; ++k) {
       dd v;
       v.hi = red[0][k];
       v.lo = red[1][k];
