@@ -303,6 +303,14 @@ struct Shape {
   int tile_y, ctas_per_sm, vec;
 };
 
+// Lattices that k_pull steps in its SMALL form: up to 300,000 padded cells, 64^3
+// and the like.  Us a step in a graph of two, without / with it, at 32 / 48 / 64 /
+// 72 stored cells a side: FP32 BGK 5.13 / 7.16 / 9.42 / 12.2 and 4.12 / 6.16 /
+// 9.25 / 12.3, LES 4.38 / 7.19 / 10.3 / 12.8 and 5.13 / 6.16 / 10.3 / 13.3 (12^3:
+// 5.14 and 4.13), FP16S BGK 6.16 / 6.34 / 9.71 / 11.3 and 4.12 / 5.15 / 7.21 / 9.61,
+// FP64 5.15 / 8.21 / 15.4 / 23.7 and 5.16 / 7.20 / 15.4 / 23.6.
+bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
+
 // Shape of a handle's steps until flb_set_launch or flb_autotune chooses one.
 // Measured on cavities (us a step at 32 / 64 / 96 / 128 / 192 / 256 / 320 stored
 // cells a side):
@@ -325,9 +333,16 @@ struct Shape {
 // at 2 / 4 cells a thread, 48 uneven blocks of 256^3 739 / 622 us, 16 cavities of
 // 32 to 128 388 / 347 us, 160^3 in blocks with LES 180 / 163 us; FP16S at 4 cells
 // 431 / 417, 262 / 259 and (MRT) 125 / 122 us; FP64 at 2 cells 1242 / 1224 us.
-// FP32S keeps one tile a CTA at 2 cells.  FP64 keeps 2 cells a thread: 1 cell and 2
-// warps took 102 / 770 us instead of 111 / 810 at 128^3 / 256^3, but 148 instead of
-// 140 us on a 143 x 162 x 120 box.
+// FP32S keeps one tile a CTA at 2 cells.
+// One block, FP32, FP32S and FP64: 2 warps a CTA, 2 cells a thread.  4 warps took
+// 107 / 390 / 198 us for 103 / 385 / 192 (FP32 BGK 160^3, 242^3, 319 x 205 x 123),
+// 474 for 457 (LES 258^3), 471 for 457 (FP32S 256^3), 428 for 419 (FP64 202^3).
+// FP64 at 1 cell took 770 instead of 800 at 256^3, but 148 instead of 140 on a
+// 143 x 162 x 120 box.  FP32 BGK whose rows are no multiple of 32 cells, above 4.5 M
+// cells: 4 cells a thread, 155 / 210 / 204 / 254 us for 162 / 223 / 223 / 315 at
+// 182^3, 202^3, 130 x 300 x 200 and 66 x 400 x 350; on aligned rows (160^3: 108 for
+// 103; 242^3: 423 for 385) and smaller lattices (152^3: 94 for 88) it loses, and MRT
+// and LES, which spill in it, lose nearly everywhere.
 Shape auto_shape(const flb_lattice* h) {
   const int storage = h->desc.storage;
   if (h->mode >= 0) {
@@ -337,7 +352,12 @@ Shape auto_shape(const flb_lattice* h) {
   const HostBlock& b = h->blocks[0];
   const long long cells = (long long)b.L.nx * b.L.ny * b.L.nz;
   const bool large = cells >= 1200000;
-  if (storage != FLB_STORAGE_FP16S) return {4, 0, 2};
+  if (storage != FLB_STORAGE_FP16S) {
+    if (small_lattice(b)) return {4, 0, 2};
+    const bool wide = storage == FLB_STORAGE_FP32 && h->desc.model == FLB_MODEL_BGK &&
+                      b.L.pitch % 32 != 0 && cells >= 4500000;
+    return {2, 0, wide ? 4 : 2};
+  }
   if (large && tma_supported(h)) return {4, -2, 4};
   return {4, 0, (h->desc.model == FLB_MODEL_MRT ? cells >= 10000000 : large) ? 4 : 2};
 }
@@ -629,14 +649,6 @@ StepParams block_half_params(const flb_lattice* h) {
   }
   return p;
 }
-
-// Lattices that k_pull steps in its SMALL form: up to 300,000 padded cells, 64^3
-// and the like.  Us a step in a graph of two, without / with it, at 32 / 48 / 64 /
-// 72 stored cells a side: FP32 BGK 5.13 / 7.16 / 9.42 / 12.2 and 4.12 / 6.16 /
-// 9.25 / 12.3, LES 4.38 / 7.19 / 10.3 / 12.8 and 5.13 / 6.16 / 10.3 / 13.3 (12^3:
-// 5.14 and 4.13), FP16S BGK 6.16 / 6.34 / 9.71 / 11.3 and 4.12 / 5.15 / 7.21 / 9.61,
-// FP64 5.15 / 8.21 / 15.4 / 23.7 and 5.16 / 7.20 / 15.4 / 23.6.
-bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 
 template <typename S, typename R, int MODEL, int V>
 void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
@@ -2071,7 +2083,7 @@ static int adjoint_backward_t(flb_lattice* h, double* dJ_dalpha, double* dJ_dtau
   FLB_CUDA(cudaGetLastError());
   int cur = 0;
   const long long chunks = (long long)(b.L.pitch / V) * b.L.ny * b.L.nz;
-  const dim3 block(32 * h->tile_y);
+  const dim3 block(32 * std::max(h->tile_y, 4));
   const dim3 grid(unsigned((chunks + block.x - 1) / block.x));
   const size_t npart = 2 * size_t(grid.x);
   if (h->adj_gpart_n < npart) {

@@ -259,3 +259,29 @@ def test_small_lattice_form_equals_the_tile_kernel(gpu_ok, storage, dims):
         out.append(lat.download_pops())
         lat.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("dims,want", [((100, 60, 50), (4, 0, 2)), ((100, 60, 51), (2, 0, 2)),
+                                       ((150, 150, 200), (2, 0, 4)), ((160, 150, 190), (2, 0, 2))])
+def test_default_fp32_shape_equals_the_tile_kernel(gpu_ok, dims, want):
+    """The shapes the library picks for FP32 BGK, on both sides of each line of
+    its rule, against the tile kernel."""
+    out = []
+    for chosen in (None, (8, 16, 2)):
+        lat = F.Lattice(*dims, 0.55)
+        flags = np.ones(dims[::-1], np.uint8)
+        flags[1:-1, 1:-1, 1:-1] = 4
+        flags[2:-2, 2:-2, 2:-2] = 2
+        flags[-2, 2:-2, 2:-2] = 8
+        lat.upload_flags(flags)
+        u = np.zeros((flags.size, 3), np.float32)
+        u[flags.reshape(-1) == 8, 0] = 0.1
+        lat.upload_field("u", u)
+        if chosen:
+            lat.set_launch(*chosen)
+        else:
+            assert lat.get_launch() == want
+        lat.step(4)
+        out.append(lat.download_pops())
+        lat.close()
+    assert np.array_equal(out[0], out[1])
