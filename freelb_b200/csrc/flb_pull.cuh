@@ -1475,17 +1475,8 @@ __global__ void k_stream_out(LayoutParams L, Geom g, H* stage, const S* pops_i, 
   }
 }
 
-// the 19 post-stream populations of cell (x,y,z)
-template <typename S, typename R>
-__device__ __forceinline__ void gather_R(const S* pops, long long dstride, const Geom& g, int x,
-                                         int y, int z, const StepParams& sp, R* f) {
-#pragma unroll
-  for (int i = 0; i < Q; ++i)
-    f[i] = Storage<S, R>::load(pops + i * dstride + wrap_src(g, x, y, z, i), sp.shift[i],
-                               sp.inv_scale);
-}
-
-// the same as stored values (FP32S: the deviations, unconverted)
+// the 19 post-stream populations of cell (x,y,z), converted (FP32S: the
+// deviations as stored)
 template <typename S, typename R>
 __device__ __forceinline__ void gather_stored(const S* pops, long long dstride, const Geom& g,
                                               int x, int y, int z, const StepParams& sp, R* v) {
