@@ -124,6 +124,7 @@ struct flb_lattice {
   long long withhold = -1; // failure-detection test hook (flb_test_withhold_tile)
   int vec = 0;  // cells per thread of the step kernel; 0 = storage default
   bool shape_chosen = false;  // by flb_set_launch or flb_autotune; else auto_shape
+  bool wide = false;  // test hook: 64-bit offsets at any size (flb_test_wide_offsets)
   int rounding = FLB_ROUND_DEFAULT;  // FP16S stores (flb_set_rounding)
   alignas(8) char snap_hdr[64] = {};  // source of the snapshot header copies
   // CUDA graphs of the two-step cycle, one per starting buffer parity
@@ -219,6 +220,11 @@ double arith_omega(const flb_lattice_desc& d, double omega) {
   return d.storage == FLB_STORAGE_FP64 ? omega : double(float(omega));
 }
 
+// Whether every element of the population arrays has a 32-bit offset.
+bool offsets32(const flb_lattice* h) {
+  return !h->wide && (long long)Q * h->dstride < (1LL << 32);
+}
+
 // Parameters shared by every kernel of the handle.
 void build_params(flb_lattice* h) {
   const flb_lattice_desc& d = h->desc;
@@ -237,7 +243,7 @@ void build_params(flb_lattice* h) {
   p.dstride = h->dstride;
   for (int i = 0; i < Q; ++i)
     p.row_off[i] = i * h->dstride - ((long long)cy(i) + (long long)cz(i) * p.ny) * p.pitch;
-  p.idx32 = h->blocks.size() == 1 && (long long)Q * h->dstride < (1LL << 32) ? 1 : 0;
+  p.idx32 = h->blocks.size() == 1 && offsets32(h) ? 1 : 0;
   for (int i = 0; i < Q; ++i) {
     p.row_off32[i] = p.idx32 ? unsigned(p.row_off[i]) : 0u;
     p.dir_off32[i] = p.idx32 ? unsigned(i * h->dstride) : 0u;
@@ -362,6 +368,15 @@ Shape auto_shape(const flb_lattice* h) {
   return {4, 0, (h->desc.model == FLB_MODEL_MRT ? cells >= 10000000 : large) ? 4 : 2};
 }
 
+// The step kernel that a handle's shape selects: the staged FP16S kernels
+// (ctas_per_sm < 0), the single-block kernel, which addresses with 32-bit offsets,
+// or the tile kernel with its block table.  A single block past 2^32 elements
+// (610^3) takes the tile kernel whatever its shape.
+bool takes_single(const flb_lattice* h) {
+  return h->mode < 0 && h->ctas_per_sm == 0 && h->sp.idx32;
+}
+bool takes_table(const flb_lattice* h) { return h->ctas_per_sm >= 0 && !takes_single(h); }
+
 Geom geom_of(const HostBlock& b) {
   return Geom{b.L.nx, b.L.ny, b.L.nz, b.L.pitch, b.L.plane, b.base};
 }
@@ -425,6 +440,9 @@ int upload_block_table(flb_lattice* h) {
   h->table_vec = vec_width(h);
   return FLB_OK;
 }
+
+// What a step of the handle's shape needs before its launches.
+int prepare_steps(flb_lattice* h) { return takes_table(h) ? upload_block_table(h) : FLB_OK; }
 
 // Host twin of wrap_src (flb_pull.cuh): P slot feeding R_i at (x,y,z).
 long long host_wrap_src(const Geom& g, int x, int y, int z, int i) {
@@ -689,10 +707,7 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
       return;
     }
   }
-  // the single-block kernel addresses with 32-bit offsets; larger lattices
-  // take the tile-table kernel
-  const bool single = h->mode < 0 && h->ctas_per_sm == 0 && h->sp.idx32;
-  if (single) {
+  if (takes_single(h)) {
     const HostBlock& b = h->blocks[0];
     const long long chunks = (long long)(b.L.pitch / V) * b.L.ny * b.L.nz;
     const long long per_cta = 32LL * h->tile_y;
@@ -718,7 +733,7 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
     long long g = h->ctas_per_sm > 0 ? (long long)h->ctas_per_sm * h->sm_count : h->ntiles;
     g = std::max(1LL, std::min(g, h->ntiles));
     if constexpr (std::is_same<S, __half>::value && V >= 2) {
-      if ((long long)Q * h->dstride < (1LL << 32)) {
+      if (offsets32(h)) {
         launch_dependent(h->dependent, k_pull_blocks_half32<MODEL, V>, unsigned(g),
                          dim3(32 * h->tile_y), 0, st, block_half_params(h), h->d_blocks,
                          h->d_tile_block, h->ntiles);
@@ -753,7 +768,7 @@ void launch_one_step(flb_lattice* h, cudaStream_t st) {
 
 template <typename S, typename R>
 int launch_steps(flb_lattice* h, int nsteps, cudaStream_t st) {
-  if (h->mode >= 0 || h->ctas_per_sm > 0) FLB_TRY(upload_block_table(h));
+  FLB_TRY(prepare_steps(h));
   h->dependent = may_depend(st);
   for (int s = 0; s < nsteps; ++s) {
     h->sp.src = h->pops[h->cur];
@@ -784,6 +799,7 @@ int launch_steps(flb_lattice* h, int nsteps, cudaStream_t st) {
 // One step from buffer src into buffer dst (adjoint recompute), leaving the
 // handle's own ping-pong state untouched.
 int step_between(flb_lattice* h, const void* src, void* dst, cudaStream_t st) {
+  FLB_TRY(prepare_steps(h));
   const void* s0 = h->sp.src;
   void* d0 = h->sp.dst;
   h->sp.src = src;
@@ -1534,7 +1550,7 @@ int flb_step_graph(flb_lattice* h, int nsteps, void* stream) {
   if (pairs > 0) {
     const int parity = h->cur;
     if (!h->graph[parity]) {
-      if (h->mode >= 0 || h->ctas_per_sm > 0) FLB_TRY(upload_block_table(h));
+      FLB_TRY(prepare_steps(h));
       cudaStream_t cap;
       FLB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
       cudaGraph_t graph = nullptr;
@@ -1625,6 +1641,19 @@ int flb_test_withhold_tile(flb_lattice* h, long long tile) {
   h->withhold = tile;
   drop_graphs(h);
   return FLB_OK;
+}
+
+int flb_test_wide_offsets(flb_lattice* h, int on) {
+  if (!h) return fail(FLB_ERR_INVALID, "null handle");
+  if (on && h->shape_chosen && h->ctas_per_sm < 0)
+    return fail(FLB_ERR_STATE, "the staged kernels address with 32-bit offsets");
+  h->wide = on != 0;
+  const StepParams keep = h->sp;
+  build_params(h);
+  h->sp.src = keep.src;
+  h->sp.dst = keep.dst;
+  drop_graphs(h);
+  return apply_auto_shape(h);
 }
 
 int flb_device_status(flb_lattice* h, void* stream) {

@@ -379,6 +379,11 @@ FLB_API int flb_get_rounding(const flb_lattice* lat, int* mode);
  * exercised without a device fault.  -1 (the default) turns it off. */
 FLB_API int flb_test_withhold_tile(flb_lattice* lat, long long tile);
 
+/* Test hook: while `on` is non-zero the handle steps as one whose populations
+ * have more than 2^32 elements, through the kernels with 64-bit offsets, so
+ * that path can be checked on a small lattice. */
+FLB_API int flb_test_wide_offsets(flb_lattice* lat, int on);
+
 /* Autotuner: times every candidate launch shape for `trial_steps` steps on
  * `stream` (CUDA events) and keeps the fastest.  The trial steps are real
  * time steps: the lattice advances by *steps_taken.  best_ms = time per step
