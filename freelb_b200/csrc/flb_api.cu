@@ -699,11 +699,9 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
       const long long ctas_needed = ((chunks + 31) / 32 + PIPE_WARPS - 1) / PIPE_WARPS;
       const long long g = std::max(1LL, std::min(ctas_needed, (long long)h->pipe_ctas * h->sm_count));
       if (pipe_wide(h))
-        launch_dependent(h->dependent, k_pull_pipe<MODEL, true>, unsigned(g), PIPE_WARPS * 32,
-                         pipe_smem_bytes(), st, h->sp);
+        k_pull_pipe<MODEL, true><<<unsigned(g), PIPE_WARPS * 32, pipe_smem_bytes(), st>>>(h->sp);
       else
-        launch_dependent(h->dependent, k_pull_pipe<MODEL, false>, unsigned(g), PIPE_WARPS * 32,
-                         pipe_smem_bytes(), st, h->sp);
+        k_pull_pipe<MODEL, false><<<unsigned(g), PIPE_WARPS * 32, pipe_smem_bytes(), st>>>(h->sp);
       return;
     }
   }
@@ -712,36 +710,36 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
     const long long chunks = (long long)(b.L.pitch / V) * b.L.ny * b.L.nz;
     const long long per_cta = 32LL * h->tile_y;
     const dim3 grid(unsigned((chunks + per_cta - 1) / per_cta));
+    const bool dependent = h->dependent && PULL_DEPENDENT<S, V>;
     if constexpr (V == 2) {
       if (small_lattice(b)) {
         if constexpr (std::is_same<S, __half>::value)
-          launch_dependent(h->dependent, k_pull<S, R, MODEL, V, true>, grid,
+          launch_dependent(dependent, k_pull<S, R, MODEL, V, true>, grid,
                            dim3(32 * h->tile_y), 0, st, half_step_params<V>(h));
         else
-          launch_dependent(h->dependent, k_pull<S, R, MODEL, V, true>, grid,
+          launch_dependent(dependent, k_pull<S, R, MODEL, V, true>, grid,
                            dim3(32 * h->tile_y), 0, st, h->sp);
         return;
       }
     }
     if constexpr (std::is_same<S, __half>::value && V >= 2)
-      launch_dependent(h->dependent, k_pull<S, R, MODEL, V>, grid,
+      launch_dependent(dependent, k_pull<S, R, MODEL, V>, grid,
                        dim3(32 * h->tile_y), 0, st, half_step_params<V>(h));
     else
-      launch_dependent(h->dependent, k_pull<S, R, MODEL, V>, grid,
+      launch_dependent(dependent, k_pull<S, R, MODEL, V>, grid,
                        dim3(32 * h->tile_y), 0, st, h->sp);
   } else {
     long long g = h->ctas_per_sm > 0 ? (long long)h->ctas_per_sm * h->sm_count : h->ntiles;
     g = std::max(1LL, std::min(g, h->ntiles));
     if constexpr (std::is_same<S, __half>::value && V >= 2) {
       if (offsets32(h)) {
-        launch_dependent(h->dependent, k_pull_blocks_half32<MODEL, V>, unsigned(g),
-                         dim3(32 * h->tile_y), 0, st, block_half_params(h), h->d_blocks,
-                         h->d_tile_block, h->ntiles);
+        k_pull_blocks_half32<MODEL, V><<<unsigned(g), dim3(32 * h->tile_y), 0, st>>>(
+            block_half_params(h), h->d_blocks, h->d_tile_block, h->ntiles);
         return;
       }
     }
-    launch_dependent(h->dependent, k_pull_blocks<S, R, MODEL, V>, unsigned(g),
-                     dim3(32 * h->tile_y), 0, st, h->sp, h->d_blocks, h->d_tile_block, h->ntiles);
+    k_pull_blocks<S, R, MODEL, V><<<unsigned(g), dim3(32 * h->tile_y), 0, st>>>(
+        h->sp, h->d_blocks, h->d_tile_block, h->ntiles);
   }
 }
 

@@ -70,10 +70,13 @@ struct StepParams {
 // its own successor start as soon as all its CTAs have (start_dependents), works
 // out its indices, and waits for everything before it on the stream to have
 // ended (wait_prerequisites) before its first load or store.  A kernel launched
-// without the attribute is ordered as usual.  Gains the launch latency between
-// steps: 100^3 FP32 37.5 -> 35.4 us a step, with the bounce-back managers of a
-// 96^3 cavity (three launches a step) 43.9 -> 39.3.  The bulk-copy kernel goes
-// without: its CTAs fill their SMs' shared memory, so none could start early.
+// without the attribute is ordered as usual.  A dependent reads what its
+// predecessors wrote with ordinary loads alone (load_word): the read-only path is
+// for memory that nobody writes while the kernel is resident.  Gains the launch
+// latency between steps: 100^3 FP32 37.5 -> 35.4 us a step, with the bounce-back
+// managers of a 96^3 cavity (three launches a step) 43.9 -> 39.3.  The bulk-copy
+// kernel goes without: its CTAs fill their SMs' shared memory, so none could start
+// early.
 __device__ __forceinline__ void start_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

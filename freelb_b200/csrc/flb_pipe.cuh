@@ -182,7 +182,7 @@ __device__ __forceinline__ void pipe_compute(const StepParams& p, const Geom& g,
         }
     }
   } else {
-    gather_words_wrap<PIPE_V>(static_cast<const __half*>(p.src), p.dstride, g, x0, int(c.y),
+    gather_words_wrap<PIPE_V, true>(static_cast<const __half*>(p.src), p.dstride, g, x0, int(c.y),
                               int(c.z), h);
   }
   const unsigned cell = c.y * unsigned(g.pitch) + c.z * unsigned(g.plane) + unsigned(x0);
@@ -205,8 +205,7 @@ __device__ __forceinline__ void pipe_compute(const StepParams& p, const Geom& g,
 template <int MODEL, bool WIDE>
 __global__ void __launch_bounds__(PIPE_WARPS * 32, FLB_PIPE_MIN_CTAS)
     k_pull_pipe(const StepParams p) {
-  start_dependents();
-  wait_prerequisites();
+  start_dependents();  // launched as usual itself: see load_word
   extern __shared__ __align__(16) unsigned char pipe_smem[];
   const int lane = int(threadIdx.x) & 31, warp = int(threadIdx.x) >> 5;
   PipeStage* st = reinterpret_cast<PipeStage*>(pipe_smem) + 2 * warp;

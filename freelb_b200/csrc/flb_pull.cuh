@@ -22,34 +22,51 @@
 
 namespace flb {
 
+// How a kernel reads its sources.  RO: through the read-only path, for kernels
+// whose sources nobody writes while they run.  A kernel launched as a dependent
+// (launch_dependent) is resident while its predecessor still writes what it will
+// read; it takes ordinary loads, which wait_prerequisites orders, through pointers
+// that promise nothing about aliasing.  k_pull with ordinary loads is as fast, but
+// for FP32 at 4 cells a thread (200^3: 227 us a step for 220); the tile kernel and
+// the pipeline spill more in FP16S (256^3 in uneven blocks: BGK 447 us for 414, MRT
+// 499 for 472; pipeline MRT 466 for 448).  Those keep the read-only path and are
+// launched as usual, which costs them 2 us a step (64^3 in blocks 16.5 for 14.6).  A
+// form of the tile kernel with ordinary loads for short steps alone rounded FP32 LES
+// differently at 2 cells a thread (other multiply-adds contracted).
+template <bool RO, typename T>
+__device__ __forceinline__ T load_word(const T* p) {
+  if constexpr (RO) return __ldg(p);
+  else return *p;
+}
+
 // V-wide aligned loads and stores of one chunk of a population array, with
 // the storage conversion of Storage<S, R> (FP16S: shift and scale).
-template <typename S, typename R, int V>
+template <typename S, typename R, int V, bool RO>
 __device__ __forceinline__ void vload(const S* p, R* out, float shift, float inv_scale) {
   if constexpr (std::is_same<S, dev32>::value) {
     // FP32S: the step and adjoint kernels work on the stored deviations
-    vload<float, R, V>(reinterpret_cast<const float*>(p), out, shift, inv_scale);
+    vload<float, R, V, RO>(reinterpret_cast<const float*>(p), out, shift, inv_scale);
   } else if constexpr (std::is_same<S, float>::value && V == 4) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 v = load_word<RO>(reinterpret_cast<const float4*>(p));
     out[0] = v.x;
     out[1] = v.y;
     out[2] = v.z;
     out[3] = v.w;
   } else if constexpr (std::is_same<S, float>::value && V == 2) {
-    const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+    const float2 v = load_word<RO>(reinterpret_cast<const float2*>(p));
     out[0] = v.x;
     out[1] = v.y;
   } else if constexpr (std::is_same<S, double>::value && V == 2) {
-    const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+    const double2 v = load_word<RO>(reinterpret_cast<const double2*>(p));
     out[0] = v.x;
     out[1] = v.y;
   } else if constexpr (std::is_same<S, __half>::value && V == 2) {
-    const unsigned v = __ldg(reinterpret_cast<const unsigned*>(p));
+    const unsigned v = load_word<RO>(reinterpret_cast<const unsigned*>(p));
     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v));
     out[0] = fmaf(a.x, inv_scale, shift);
     out[1] = fmaf(a.y, inv_scale, shift);
   } else if constexpr (std::is_same<S, __half>::value && V == 4) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 v = load_word<RO>(reinterpret_cast<const uint2*>(p));
     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
     const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
     out[0] = fmaf(a.x, inv_scale, shift);
@@ -160,8 +177,8 @@ __device__ __forceinline__ bool interior_row(const Geom& g, int y, int z) {
 // ROWS: the wrap rule on linear rows (wrap_row_off), straight-line code whose
 // loads are all in flight together; the cell-wise rule branches from load to
 // load, but needs fewer registers.
-template <typename S, typename R, int V, int SIGN, bool ROWS = false>
-__device__ __forceinline__ void gather_chunk(const S* __restrict__ arr, long long dstride,
+template <typename S, typename R, int V, int SIGN, bool RO = true, bool ROWS = false>
+__device__ __forceinline__ void gather_chunk(const S* arr, long long dstride,
                                              const Geom& g, const float* shift, float inv_scale,
                                              int x0, int y, int z, R (&vals)[Q][V]) {
   const bool active = true;
@@ -175,19 +192,19 @@ __device__ __forceinline__ void gather_chunk(const S* __restrict__ arr, long lon
       const S* rowp = arr + i * dstride + g.base + (long long)(y - ey) * g.pitch +
                       (long long)(z - ez) * g.plane;
       R v[V];
-      vload<S, R, V>(rowp + xl, v, shift[i], inv_scale);
+      vload<S, R, V, RO>(rowp + xl, v, shift[i], inv_scale);
       if (ex == 0) {
 #pragma unroll
         for (int k = 0; k < V; ++k) vals[i][k] = v[k];
       } else if (ex > 0) {
         R w[V];  // chunk before: its last element is x0 - 1
-        vload<S, R, V>(rowp + xprev, w, shift[i], inv_scale);
+        vload<S, R, V, RO>(rowp + xprev, w, shift[i], inv_scale);
         vals[i][0] = w[V - 1];
 #pragma unroll
         for (int k = 1; k < V; ++k) vals[i][k] = v[k - 1];
       } else {
         R w[V];  // chunk after: its first element is x0 + V
-        vload<S, R, V>(rowp + xnext, w, shift[i], inv_scale);
+        vload<S, R, V, RO>(rowp + xnext, w, shift[i], inv_scale);
 #pragma unroll
         for (int k = 0; k < V - 1; ++k) vals[i][k] = v[k + 1];
         vals[i][V - 1] = w[0];
@@ -291,18 +308,18 @@ template <int V> struct HWord;
 template <> struct HWord<2> { using type = unsigned; };
 template <> struct HWord<4> { using type = uint2; };
 
-template <int V>
+template <int V, bool RO>
 __device__ __forceinline__ typename HWord<V>::type hload(const __half* p) {
-  if constexpr (V == 4) return __ldg(reinterpret_cast<const uint2*>(p));
-  else return __ldg(reinterpret_cast<const unsigned*>(p));
+  return load_word<RO>(reinterpret_cast<const typename HWord<V>::type*>(p));
 }
 template <int V>
 __device__ __forceinline__ void hstore(__half* p, const typename HWord<V>::type& w) {
   if constexpr (V == 4) *reinterpret_cast<uint2*>(p) = w;
   else *reinterpret_cast<unsigned*>(p) = w;
 }
+template <bool RO>
 __device__ __forceinline__ unsigned hscalar(const __half* p) {
-  return __ldg(reinterpret_cast<const unsigned short*>(p));
+  return load_word<RO>(reinterpret_cast<const unsigned short*>(p));
 }
 // 32-bit part holding halves k and k+1 (k even) of a word
 __device__ __forceinline__ unsigned& hpart(unsigned& w, int) { return w; }
@@ -338,10 +355,10 @@ __device__ __forceinline__ uint2 hsplice_next(uint2 v, uint2 w) {
 // components per D3Q19 velocity the carry reaches z only when the y row wraps,
 // and then c_z = 0.
 // Rows near the block's first and last planes: every source through the wrap rule.
-template <int V, bool ROWS = false>
-__device__ __forceinline__ void gather_words_wrap(const __half* __restrict__ arr,
-                                                  long long dstride, const Geom& g, int x0,
-                                                  int y, int z, typename HWord<V>::type (&h)[Q]) {
+template <int V, bool RO, bool ROWS = false>
+__device__ __forceinline__ void gather_words_wrap(const __half* arr, long long dstride,
+                                                  const Geom& g, int x0, int y, int z,
+                                                  typename HWord<V>::type (&h)[Q]) {
   using W = typename HWord<V>::type;
 #pragma unroll
   for (int i = 0; i < Q; ++i) h[i] = W{};
@@ -351,7 +368,7 @@ __device__ __forceinline__ void gather_words_wrap(const __half* __restrict__ arr
 #pragma unroll
     for (int i = 0; i < Q; ++i)
       hset(h[i], k,
-           hscalar(arr + i * dstride +
+           hscalar<RO>(arr + i * dstride +
                    (ROWS ? wrap_row_off(g, x, z * g.ny + y, -cx(i), -(cy(i) + g.ny * cz(i)))
                          : wrap_off(g, x, y, z, -cx(i), -cy(i), -cz(i)))));
   }
@@ -370,20 +387,20 @@ __device__ __forceinline__ void gather_words_dir(const StepParams& p, const Geom
 #pragma unroll
   for (int i = 0; i < Q; ++i) {
     const __half* own = static_cast<const __half*>(p.src_dir[i]) + cell;
-    const W v = hload<V>(own);
+    const W v = hload<V, false>(own);
     if (cx(i) == 0) {
       h[i] = v;
     } else if (cx(i) > 0) {
-      h[i] = hsplice_prev(hload<V>(own - V), v);
+      h[i] = hsplice_prev(hload<V, false>(own - V), v);
     } else {
-      h[i] = hsplice_next(v, hload<V>(own + V));
+      h[i] = hsplice_next(v, hload<V, false>(own + V));
     }
   }
   if (x0 == 0) {  // x = nx-1 of the row before the source row
     const unsigned e = cell - unsigned(g.pitch) + unsigned(g.nx - 1);
 #pragma unroll
     for (int i = 1; i < Q; ++i)
-      if (cx(i) > 0) hset(h[i], 0, hscalar(static_cast<const __half*>(p.src_dir[i]) + e));
+      if (cx(i) > 0) hset(h[i], 0, hscalar<false>(static_cast<const __half*>(p.src_dir[i]) + e));
   }
   const int klast = g.nx - 1 - x0;
   if (klast >= 0 && klast < V) {  // x = 0 of the row after the source row
@@ -391,7 +408,7 @@ __device__ __forceinline__ void gather_words_dir(const StepParams& p, const Geom
 #pragma unroll
     for (int i = 1; i < Q; ++i)
       if (cx(i) < 0) {
-        const unsigned w = hscalar(static_cast<const __half*>(p.src_dir[i]) + e);
+        const unsigned w = hscalar<false>(static_cast<const __half*>(p.src_dir[i]) + e);
 #pragma unroll
         for (int k = 0; k < V; ++k)
           if (k == klast) hset(h[i], k, w);
@@ -415,33 +432,33 @@ __device__ __forceinline__ void gather_words(const __half* __restrict__ arr, lon
       rowp[i] = row + (row_off ? row_off[i]
                                : i * dstride - (long long)cy(i) * g.pitch -
                                      (long long)cz(i) * g.plane);
-      const W v = hload<V>(rowp[i] + x0);
+      const W v = hload<V, true>(rowp[i] + x0);
       if (cx(i) == 0) {
         h[i] = v;
       } else if (cx(i) > 0) {
-        h[i] = hsplice_prev(hload<V>(rowp[i] + xprev), v);
+        h[i] = hsplice_prev(hload<V, true>(rowp[i] + xprev), v);
       } else {
-        h[i] = hsplice_next(v, hload<V>(rowp[i] + xnext));
+        h[i] = hsplice_next(v, hload<V, true>(rowp[i] + xnext));
       }
     }
     if (x0 == 0) {  // x = nx-1 of the row before the source row
 #pragma unroll
       for (int i = 1; i < Q; ++i)
-        if (cx(i) > 0) hset(h[i], 0, hscalar(rowp[i] - g.pitch + (g.nx - 1)));
+        if (cx(i) > 0) hset(h[i], 0, hscalar<true>(rowp[i] - g.pitch + (g.nx - 1)));
     }
     const int klast = g.nx - 1 - x0;
     if (klast >= 0 && klast < V) {  // x = 0 of the row after the source row
 #pragma unroll
       for (int i = 1; i < Q; ++i)
         if (cx(i) < 0) {
-          const unsigned e = hscalar(rowp[i] + g.pitch);
+          const unsigned e = hscalar<true>(rowp[i] + g.pitch);
 #pragma unroll
           for (int k = 0; k < V; ++k)
             if (k == klast) hset(h[i], k, e);
         }
     }
   } else {
-    gather_words_wrap<V>(arr, dstride, g, x0, y, z, h);
+    gather_words_wrap<V, true>(arr, dstride, g, x0, y, z, h);
   }
 }
 
@@ -1216,7 +1233,7 @@ __device__ __forceinline__ void pull_chunk_half32(const StepParams& p, const Geo
     gather_words_dir<V>(p, g, x0, cell, h);
   } else {
     const unsigned z = row / unsigned(g.ny);
-    gather_words_wrap<V, ROWS>(static_cast<const __half*>(p.src), p.dstride, g, x0,
+    gather_words_wrap<V, false, ROWS>(static_cast<const __half*>(p.src), p.dstride, g, x0,
                                int(row - z * unsigned(g.ny)), int(z), h);
   }
   uint8_t fl[V];
@@ -1246,13 +1263,13 @@ __device__ __forceinline__ void gather_words_blk(const StepParams& p, const Geom
   for (int i = 0; i < Q; ++i) {
     const unsigned sc = cell - unsigned(cy(i)) * pitch - unsigned(cz(i)) * plane;
     const __half* own = static_cast<const __half*>(p.src_dir[i]) + sc;
-    const W v = hload<V>(own);
+    const W v = hload<V, true>(own);
     if (cx(i) == 0) {
       h[i] = v;
     } else if (cx(i) > 0) {
-      h[i] = hsplice_prev(hload<V>(x0 >= V ? own - V : own), v);
+      h[i] = hsplice_prev(hload<V, true>(x0 >= V ? own - V : own), v);
     } else {
-      h[i] = hsplice_next(v, hload<V>(x0 + V < g.nx ? own + V : own));
+      h[i] = hsplice_next(v, hload<V, true>(x0 + V < g.nx ? own + V : own));
     }
   }
   if (x0 == 0) {  // x = nx-1 of the row before the source row
@@ -1261,7 +1278,7 @@ __device__ __forceinline__ void gather_words_blk(const StepParams& p, const Geom
       if (cx(i) > 0) {
         const unsigned e = cell - unsigned(cy(i)) * pitch - unsigned(cz(i)) * plane - pitch +
                            unsigned(g.nx - 1);
-        hset(h[i], 0, hscalar(static_cast<const __half*>(p.src_dir[i]) + e));
+        hset(h[i], 0, hscalar<true>(static_cast<const __half*>(p.src_dir[i]) + e));
       }
   }
   const int klast = g.nx - 1 - x0;
@@ -1271,7 +1288,7 @@ __device__ __forceinline__ void gather_words_blk(const StepParams& p, const Geom
       if (cx(i) < 0) {
         const unsigned e = cell - unsigned(cy(i)) * pitch - unsigned(cz(i)) * plane + pitch -
                            unsigned(x0);
-        const unsigned w = hscalar(static_cast<const __half*>(p.src_dir[i]) + e);
+        const unsigned w = hscalar<true>(static_cast<const __half*>(p.src_dir[i]) + e);
 #pragma unroll
         for (int k = 0; k < V; ++k)
           if (k == klast) hset(h[i], k, w);
@@ -1288,7 +1305,7 @@ __device__ __forceinline__ void pull_chunk_half_blk32(const StepParams& p, const
   if (interior_row(g, y, z))
     gather_words_blk<V>(p, g, x0, cell, h);
   else
-    gather_words_wrap<V>(static_cast<const __half*>(p.src), p.dstride, g, x0, y, z, h);
+    gather_words_wrap<V, true>(static_cast<const __half*>(p.src), p.dstride, g, x0, y, z, h);
   uint8_t fl[V];
   load_flags<V>(p.flags + cell, fl);
   collide_half<MODEL, V>(p, omega, (long long)cell, fl, h);
@@ -1296,17 +1313,17 @@ __device__ __forceinline__ void pull_chunk_half_blk32(const StepParams& p, const
   for (int i = 0; i < Q; ++i) hstore<V>(static_cast<__half*>(p.dst_dir[i]) + cell, h[i]);
 }
 
-template <typename S, typename R, int MODEL, int V, bool ROWS = false>
+template <typename S, typename R, int MODEL, int V, bool RO = true, bool ROWS = false>
 __device__ __forceinline__ void pull_chunk(const StepParams& p, const Geom& g, R omega, int lane,
                                            int x0, int y, int z) {
   if constexpr (std::is_same<S, __half>::value && V >= 2) {
     pull_chunk_half<MODEL, V>(p, g, omega, x0, y, z);
     return;
   }
-  const S* __restrict__ src = static_cast<const S*>(p.src);
+  const S* src = static_cast<const S*>(p.src);
   S* __restrict__ dst = static_cast<S*>(p.dst);
   R vals[Q][V];
-  gather_chunk<S, R, V, 1, ROWS>(src, p.dstride, g, p.shift, p.inv_scale, x0, y, z, vals);
+  gather_chunk<S, R, V, 1, RO, ROWS>(src, p.dstride, g, p.shift, p.inv_scale, x0, y, z, vals);
   const int nvalid = min(V, g.nx - x0);
   const long long cell0 = g.base + (long long)y * g.pitch + (long long)z * g.plane + x0;
   uint8_t fl[V];
@@ -1374,7 +1391,12 @@ struct PullBounds {
                                                               : 3;
 };
 
-//
+// Forms of k_pull that may be launched as dependents: those that lose nothing with
+// ordinary loads (load_word).
+template <typename S, int V>
+constexpr bool PULL_DEPENDENT =
+    !((std::is_same<S, float>::value || std::is_same<S, dev32>::value) && V == 4);
+
 // SMALL: lattices that do not fill the GPU (small_lattice in flb_api.cu), where
 // a step takes as long as one thread's chain of work.  The longest chain is that
 // of the rows near the first and last planes, so it takes the straight-line wrap
@@ -1400,19 +1422,21 @@ __global__ void __launch_bounds__(256, SMALL ? 1 : PullBounds<S, MODEL, V>::min_
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int x0, y, z;
   if (!chunk_coords<V>(g, q, x0, y, z)) return;
-  wait_prerequisites();
-  pull_chunk<S, R, MODEL, V, SMALL>(p, g, R(p.omega), 0, x0, y, z);
+  constexpr bool RO = !PULL_DEPENDENT<S, V>;
+  if constexpr (!RO) wait_prerequisites();
+  pull_chunk<S, R, MODEL, V, RO, SMALL>(p, g, R(p.omega), 0, x0, y, z);
 }
 
 // Many blocks: tiles of blockDim.x consecutive chunks, numbered block by block
 // (tile_start = first tile of the block, tile_block = block of every tile);
 // CTAs walk the tiles with a grid stride (persistent) or take one tile each.
+// Launched as usual, so its sources are its own alone (load_word); the halo copies
+// after it may start early.
 template <typename S, typename R, int MODEL, int V>
 __global__ void __launch_bounds__(256, PullBounds<S, MODEL, V>::min_ctas)
     k_pull_blocks(const StepParams p, const BlockEntry* __restrict__ blocks,
                   const int* __restrict__ tile_block, long long ntiles) {
   start_dependents();
-  wait_prerequisites();
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BlockEntry& b = blocks[__ldg(tile_block + t)];
     const long long q = (t - b.tile_start) * blockDim.x + threadIdx.x;
@@ -1428,7 +1452,6 @@ __global__ void __launch_bounds__(256, PullBounds<__half, MODEL, V>::min_ctas)
     k_pull_blocks_half32(const StepParams p, const BlockEntry* __restrict__ blocks,
                          const int* __restrict__ tile_block, long long ntiles) {
   start_dependents();
-  wait_prerequisites();
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BlockEntry& b = blocks[__ldg(tile_block + t)];
     const long long q = (t - b.tile_start) * blockDim.x + threadIdx.x;

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import freelb_b200 as F
+from freelb_b200 import geometry
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +63,54 @@ def test_steps_captured_by_the_caller(gpu_ok, storage):
     torch.cuda.synchronize()
     b.step(10)
     assert np.array_equal(a.download_pops(), b.download_pops())
+
+
+def shaped(storage, model, ni, shape):
+    lat = F.cavity(ni, tau=0.55, storage=storage, model=model)
+    lat.set_launch(*shape)
+    return lat
+
+
+def blocks(storage, model):
+    """A cavity of 98^3 in blocks with halos, in the shape the library picks."""
+    ni = 96
+    parts = geometry.uneven_blocks(ni, edges=(32, 48), seed=1)
+    lat = F.Lattice.blocks(geometry.block_tuples(parts), 0.55, mode="halo", storage=storage,
+                           model=model)
+    flags = F.cavity_flags(ni)
+    u = np.zeros((flags.size, 3))
+    u[flags == 8, 0] = 0.1
+    for k, b in enumerate(parts):
+        lat.upload_flags(geometry.slice_block(flags, ni + 2, b), block=k)
+        lat.upload_field("u", geometry.slice_block(u, ni + 2, b, comps=3), block=k)
+    return lat
+
+
+WIDE, PERSISTENT, PIPELINE = (2, 0, 4), (4, 8, 2), (4, -1, 4)
+
+
+@pytest.mark.parametrize("make", [
+    lambda: shaped("fp32", "bgk", 148, WIDE), lambda: shaped("fp32", "mrt", 148, (4, 0, 2)),
+    lambda: shaped("fp32", "les", 126, PERSISTENT), lambda: shaped("fp32s", "bgk", 126, (4, 0, 2)),
+    lambda: shaped("fp64", "bgk", 126, (4, 0, 2)), lambda: shaped("fp16s", "bgk", 148, WIDE),
+    lambda: shaped("fp16s", "mrt", 126, (4, 0, 2)), lambda: shaped("fp16s", "bgk", 126, PIPELINE),
+    lambda: shaped("fp16s", "les", 148, PIPELINE), lambda: blocks("fp32", "bgk"),
+    lambda: blocks("fp16s", "bgk"), lambda: blocks("fp64", "bgk"), lambda: blocks("fp32s", "bgk"),
+])
+def test_every_step_kernel_keeps_its_order(gpu_ok, make):
+    """Each form of the step that may start early, on lattices of several waves of
+    CTAs, and the halo copies after it: 24 steps in a row against 24 waited for."""
+    import torch
+    out = []
+    for wait in (False, True):
+        lat = make()
+        torch.cuda.synchronize()
+        if wait:
+            for _ in range(24):
+                lat.step(1)
+                torch.cuda.synchronize()
+        else:
+            lat.step(24)
+        out.append([lat.download_pops(block=b) for b in range(lat.nblocks)])
+        lat.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
