@@ -121,6 +121,7 @@ struct flb_lattice {
   int pipe_ctas = 0;    // resident k_pull_pipe CTAs per SM (0 = not yet queried)
   bool tma_ready = false;  // k_pull_tma shared-memory attributes set
   double wait_s = 2.0;     // bound of one device-side wait (k_pull_tma)
+  bool waits = false;      // a kernel with bounded waits was launched (k_pull_tma)
   long long withhold = -1; // failure-detection test hook (flb_test_withhold_tile)
   int vec = 0;  // cells per thread of the step kernel; 0 = storage default
   bool shape_chosen = false;  // by flb_set_launch or flb_autotune; else auto_shape
@@ -158,6 +159,22 @@ void drop_graphs(flb_lattice* h) {
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
+}
+
+int report_wait(int status) {
+  return fail(status, "a device-side wait gave up (status %d): the steps since the last "
+                      "flb_device_status are incomplete", status);
+}
+
+// End of a call that hands results to the host: wait for the stream, and report a
+// wait of the steps before that gave up.  The bulk-copy kernel is a default, so a
+// caller may have chosen no shape and has no reason to ask for the status.
+int finish(flb_lattice* h, cudaStream_t st) {
+  int v = 0;
+  if (h->waits)
+    FLB_CUDA(cudaMemcpyAsync(&v, status_word(h), sizeof v, cudaMemcpyDeviceToHost, st));
+  FLB_CUDA(cudaStreamSynchronize(st));
+  return v == 0 ? FLB_OK : report_wait(v);
 }
 
 int ensure_stage(flb_lattice* h, size_t bytes) {
@@ -675,6 +692,7 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
       const HostBlock& b = h->blocks[0];
       const int cv = h->ctas_per_sm == -2 ? 2 : 4;
       const long long cells = (long long)cv * TMA_CHUNKS;
+      h->waits = true;
       TmaParams tp{};
       tp.ntiles = (b.padded() + cells - 1) / cells;
       tp.status = status_word(h);
@@ -870,6 +888,7 @@ int pops_transfer(flb_lattice* h, const HostBlock& B, void* host, bool upload, c
     }
     FLB_CUDA(cudaGetLastError());
   }
+  if (!upload) return finish(h, st);
   FLB_CUDA(cudaStreamSynchronize(st));
   return FLB_OK;
 }
@@ -923,6 +942,7 @@ int field_transfer(flb_lattice* h, const HostBlock& B, int field, void* host, bo
     return fail(FLB_ERR_INVALID, "unknown field %d", field);
   }
   FLB_CUDA(cudaGetLastError());
+  if (!upload) return finish(h, st);
   FLB_CUDA(cudaStreamSynchronize(st));
   return FLB_OK;
 }
@@ -1663,8 +1683,7 @@ int flb_device_status(flb_lattice* h, void* stream) {
   if (v == 0) return FLB_OK;
   FLB_CUDA(cudaMemsetAsync(status_word(h), 0, sizeof v, st));
   FLB_CUDA(cudaStreamSynchronize(st));
-  return fail(v, "a device-side wait gave up (status %d): the steps since the last check "
-                 "are incomplete", v);
+  return report_wait(v);
 }
 
 int flb_get_launch(const flb_lattice* h, int* tile_y, int* ctas_per_sm, int* cells_per_thread) {
@@ -1757,6 +1776,7 @@ int flb_autotune(flb_lattice* h, int trial_steps, void* stream, int* tile_y, int
       }
     }
   }
+  if (!rc) rc = finish(h, st);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) {
@@ -1807,8 +1827,7 @@ int flb_reduce_conservation(flb_lattice* h, uint8_t key, double out[4], void* st
   }));
   FLB_CUDA(cudaGetLastError());
   FLB_CUDA(cudaMemcpyAsync(out, h->acc, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  FLB_CUDA(cudaStreamSynchronize(st));
-  return FLB_OK;
+  return finish(h, st);
 }
 
 int flb_tolerance_u(flb_lattice* h, uint8_t key, double* max_du, void* stream) {
@@ -1833,7 +1852,7 @@ int flb_tolerance_u(flb_lattice* h, uint8_t key, double* max_du, void* stream) {
   FLB_CUDA(cudaGetLastError());
   unsigned long long bits = 0;
   FLB_CUDA(cudaMemcpyAsync(&bits, acc, sizeof bits, cudaMemcpyDeviceToHost, st));
-  FLB_CUDA(cudaStreamSynchronize(st));
+  FLB_TRY(finish(h, st));
   std::memcpy(max_du, &bits, sizeof(double));
   return FLB_OK;
 }
@@ -1855,7 +1874,7 @@ int flb_check_finite(flb_lattice* h, uint64_t* bad, void* stream) {
   FLB_CUDA(cudaGetLastError());
   unsigned long long v = 0;
   FLB_CUDA(cudaMemcpyAsync(&v, acc, sizeof v, cudaMemcpyDeviceToHost, st));
-  FLB_CUDA(cudaStreamSynchronize(st));
+  FLB_TRY(finish(h, st));
   *bad = v;
   if (v) return fail(FLB_ERR_NUMERIC, "%llu non-finite populations", v);
   return FLB_OK;
@@ -2273,7 +2292,7 @@ int flb_vtk_field_base64(flb_lattice* h, int block, int field, int overlap, int 
   else rc = vtk_launch<float, float>(a, d_out, st);
   cudaError_t e = cudaSuccess;
   if (rc == FLB_OK) e = cudaMemcpyAsync(out, d_out, nchar, cudaMemcpyDeviceToHost, st);
-  if (rc == FLB_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (rc == FLB_OK && e == cudaSuccess) rc = finish(h, st);
   cudaFree(d_out);
   if (rc) return rc;
   if (e != cudaSuccess)

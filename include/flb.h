@@ -320,8 +320,7 @@ FLB_API int flb_download_field_block(flb_lattice* lat, int block, int field, voi
  * one thread stages each tile's 19 source ranges and flags in shared memory
  * with bulk asynchronous copies (3 / 5 stages) while 15 warps collide the
  * staged tiles; 4 cells per thread (cells_per_thread 4 or 0; the staged
- * warps run 2-cell chunks).  Its waits are bounded (flb_set_wait_limit;
- * flb_device_status reports one that gave up).
+ * warps run 2-cell chunks).  Its waits are bounded (flb_set_wait_limit).
  * Without a call the library picks a shape by storage, model and size
  * (flb_get_launch tells which): small FP16S lattices 2 cells per thread, large
  * ones the bulk-copy kernel where the rows suit it, multi-block handles a
@@ -337,7 +336,11 @@ FLB_API int flb_get_launch(const flb_lattice* lat, int* tile_y, int* ctas_per_sm
  * and the kernel ends early, leaving that step incomplete.
  * flb_set_wait_limit sets the bound of one wait (seconds, default 2, at most
  * 60).  flb_device_status synchronises `stream` and returns FLB_OK, or the
- * recorded code (which it clears). */
+ * recorded code (which it clears).  Until then the calls that synchronise to
+ * hand results to the host return the code too: downloads of populations and
+ * fields, flb_reduce_conservation, flb_tolerance_u, flb_check_finite,
+ * flb_vtk_field_base64 and flb_autotune.  Calls that only enqueue work
+ * (flb_step, flb_compute_rhou, flb_snapshot_save) do not look. */
 FLB_API int flb_set_wait_limit(flb_lattice* lat, double seconds);
 FLB_API int flb_device_status(flb_lattice* lat, void* stream);
 /* Population snapshots (checkpoint / resume; no reference counterpart: FreeLB

@@ -146,6 +146,34 @@ def test_tma_wait_that_gives_up_is_reported_and_the_handle_recovers(gpu_ok):
     assert np.array_equal(lat.download_pops(), ref.download_pops())
 
 
+def test_results_of_a_default_handle_report_a_wait_that_gave_up(gpu_ok):
+    """A caller who chose no launch shape runs the bulk-copy kernel at 110^3: until
+    the status is read, every call that brings results to the host reports the
+    incomplete step, and uploads, the way back, do not."""
+    lat = F.cavity(108, tau=0.55, storage="fp16s")
+    assert lat.get_launch() == (4, -2, 4)
+    start = lat.download_pops(np.float64)
+    lat.set_wait_limit(0.05)
+    F._capi.call("flb_test_withhold_tile", lat._h, 150)
+    lat.step(1)
+    F._capi.call("flb_test_withhold_tile", lat._h, -1)
+    lat.compute_rhou(2)
+    for call in (lat.download_pops, lambda: lat.download_field("rho"),
+                 lambda: lat.download_field("u"), lambda: lat.conservation(2),
+                 lambda: lat.tolerance_u(2), lat.nonfinite, lambda: lat.autotune(1),
+                 lambda: lat.vtk_body("rho")):
+        with pytest.raises(F.FlbError) as e:
+            call()
+        assert e.value.code == -4      # FLB_ERR_TIMEOUT
+    assert lat.get_launch() == (4, -2, 4)
+    lat.upload_pops(start)
+    with pytest.raises(F.FlbError):
+        lat.device_status()
+    lat.set_wait_limit(2.0)
+    assert np.array_equal(lat.download_pops(np.float64), start)
+    assert lat.conservation(2)[0] > 0
+
+
 @pytest.mark.parametrize("ni,model,want", [
     (104, "bgk", (4, 0, 2)),    # 106^3: the last size below the line
     (106, "bgk", (4, 0, 4)),    # 108^3: above it, rows not on 16-byte boundaries
