@@ -1705,6 +1705,7 @@ int flb_autotune(flb_lattice* h, int trial_steps, void* stream, int* tile_y, int
   const int vecs_d[] = {1, 2}, vecs_f[] = {2, 4};
   const int* vecs = h->desc.storage == FLB_STORAGE_FP64 ? vecs_d : vecs_f;
   const int ty0 = h->tile_y, c0 = h->ctas_per_sm, v0 = vec_width(h);
+  const bool chosen0 = h->shape_chosen;
   int best_ty = ty0, best_c = c0, best_v = v0, taken = 0;
   float best = 1e30f;
   cudaEvent_t e0, e1;
@@ -1780,7 +1781,10 @@ int flb_autotune(flb_lattice* h, int trial_steps, void* stream, int* tile_y, int
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) {
+    const std::string why = g_err;
     flb_set_launch(h, ty0, c0, v0);
+    h->shape_chosen = chosen0;
+    g_err = why;
     return rc;
   }
   FLB_TRY(flb_set_launch(h, best_ty, best_c, best_v));

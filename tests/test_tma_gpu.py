@@ -4,6 +4,8 @@ and collided there.  It must give the direct kernel's bits on every cell, for
 every model, on lattices whose tiles fall across row ends, padding and the
 unstaged tiles near the first and last planes; its bounded waits must report a
 wait that gave up through flb_device_status, and leave the handle usable."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -184,7 +186,7 @@ def test_results_of_a_default_handle_report_a_wait_that_gave_up(gpu_ok):
 ])
 def test_default_shape_gives_the_direct_kernels_bits(gpu_ok, ni, model, want):
     """The shape the library picks by itself, on both sides of each line of its
-    rule, and the one it picks again when the model changes."""
+    rule."""
     a, b = (F.cavity(ni, tau=0.55, storage="fp16s", model=model) for _ in range(2))
     assert a.get_launch() == want
     b.set_launch(1, 0, 4)
@@ -192,3 +194,40 @@ def test_default_shape_gives_the_direct_kernels_bits(gpu_ok, ni, model, want):
     b.step(6)
     a.device_status()
     assert np.array_equal(a.download_pops(), b.download_pops())
+
+
+def set_model(lat, model):
+    keys = (ctypes.c_uint8 * 3)(2, 4, 8)
+    ops = (ctypes.c_uint8 * 3)(F._capi.OP_BULK, F._capi.OP_BOUNCEBACK, F._capi.OP_MOVINGWALL)
+    F._capi.call("flb_set_tasks", lat._h, 3, keys, ops, model)
+
+
+def test_default_shape_follows_the_model_of_a_live_handle(gpu_ok):
+    """108^3 stored cells, whose rows do not suit the bulk copies: MRT takes 2 cells a
+    thread there and BGK 4.  A handle that changes its model gives the bits of one
+    whose shape is chosen; a tuning run that fails chooses nothing."""
+    a, b = (F.cavity(106, tau=0.55, storage="fp16s", model="mrt") for _ in range(2))
+    b.set_launch(1, 0, 4)
+    for model, want in ((F._capi.MODEL_BGK, (4, 0, 4)), (F._capi.MODEL_MRT, (4, 0, 2)),
+                        (F._capi.MODEL_BGK, (4, 0, 4))):
+        set_model(a, model)
+        set_model(b, model)
+        assert a.get_launch() == want and b.get_launch() == (1, 0, 4)
+        a.step(4)
+        b.step(4)
+        assert np.array_equal(a.download_pops(), b.download_pops())
+
+
+def test_failed_autotune_leaves_the_default_in_charge(gpu_ok):
+    lat = F.cavity(108, tau=0.55, storage="fp16s", model="mrt")
+    lat.set_wait_limit(0.05)
+    F._capi.call("flb_test_withhold_tile", lat._h, 150)
+    lat.step(1)
+    F._capi.call("flb_test_withhold_tile", lat._h, -1)
+    with pytest.raises(F.FlbError) as e:
+        lat.autotune(1)
+    assert e.value.code == -4 and "gave up" in str(e.value)
+    lat.set_wait_limit(2.0)
+    assert lat.get_launch() == (4, -2, 4)
+    F._capi.call("flb_test_wide_offsets", lat._h, 1)    # the default shape is picked again
+    assert lat.get_launch() == (4, 0, 2)
