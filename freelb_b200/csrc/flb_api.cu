@@ -1788,6 +1788,7 @@ int flb_autotune(flb_lattice* h, int trial_steps, void* stream, int* tile_y, int
     return rc;
   }
   FLB_TRY(flb_set_launch(h, best_ty, best_c, best_v));
+  FLB_TRY(prepare_steps(h));  // the winner's table, not that of the last shape timed
   if (tile_y) *tile_y = best_ty;
   if (ctas_per_sm) *ctas_per_sm = best_c;
   if (cells_per_thread) *cells_per_thread = best_v;

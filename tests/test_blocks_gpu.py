@@ -285,3 +285,20 @@ def test_default_fp32_shape_equals_the_tile_kernel(gpu_ok, dims, want):
         out.append(lat.download_pops())
         lat.close()
     assert np.array_equal(out[0], out[1])
+
+
+def test_autotune_leaves_the_winner_ready_to_be_captured(gpu_ok):
+    """After a tuning run the block table is that of the shape it kept, so a
+    caller's capture of the next steps allocates and copies nothing."""
+    import torch
+    a, b = (gpu_blocks(40, G.uneven_blocks(40, edges=(8, 12, 16), seed=2)) for _ in range(2))
+    taken = a.autotune(trial_steps=1)[2]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        a.step(2, stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    b.step(taken + 2)
+    for k in range(a.nblocks):
+        assert np.array_equal(a.download_pops(block=k), b.download_pops(block=k))
