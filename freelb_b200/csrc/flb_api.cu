@@ -320,6 +320,7 @@ bool vec_allowed(int storage, int v) {
   return storage == FLB_STORAGE_FP64 ? (v == 1 || v == 2) : (v == 2 || v == 4);
 }
 bool tma_supported(const flb_lattice* h);
+bool use_mrt2(const flb_lattice* h);
 
 // Launch shape of one step.
 struct Shape {
@@ -352,11 +353,36 @@ bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 // sides meet between 96^3 and 128^3.  Where the rows do not suit the bulk
 // copies, BGK and LES change to 4 cells a thread there and MRT (whose 4-cell
 // form spills) at 10 M cells (between 192^3 and 256^3).
-// Many blocks (4 warps each; one tile a CTA / persistent, 32 CTAs an SM): FP32
-// at 2 / 4 cells a thread, 48 uneven blocks of 256^3 739 / 622 us, 16 cavities of
-// 32 to 128 388 / 347 us, 160^3 in blocks with LES 180 / 163 us; FP16S at 4 cells
-// 431 / 417, 262 / 259 and (MRT) 125 / 122 us; FP64 at 2 cells 1242 / 1224 us.
-// FP32S keeps one tile a CTA at 2 cells.
+// Many blocks, 4 warps a CTA.  Us a step of persistent grids (32 CTAs an SM) at the
+// larger number of cells a thread / one tile a CTA, the same / one tile a CTA at 2
+// cells (FP64: 1), for cavities of 48 / 64 / 96 / 128 / 160 / 256 cells a side in uneven
+// blocks (0.13 / 0.31 / 0.98 / 2.4 / 4.6 / 18.8 M padded cells), then 4 (0.51 M) and 16
+// (11.6 M) independent ones:
+//   FP32 BGK     12.2 / 16.8 / 42.5 / 96.7 / 161 / 674, 18.7, 342
+//                12.1 / 16.6 / 39.4 / 89.0 / 150 / 626, 18.5, 318
+//                 8.4 / 14.6 / 39.7 / 101 / 174 / 742, 18.6, 366
+//   FP32 LES     12.5 / 18.0 / 43.6 / 104 / 177 / 756, 20.4, 391
+//                12.4 / 17.5 / 43.1 / 101 / 172 / 705, 19.8, 372
+//                 8.7 / 16.5 / 42.5 / 105 / 180 / 768, 20.6, 383
+//   FP32 MRT     12.5 / 17.8 / 41.2 / 94.5 / 159 / 667, 19.4, 341
+//   (two-rate)   12.5 / 17.4 / 41.2 / 94.8 / 162 / 666, 19.3, 344
+//                10.1 / 16.6 / 43.2 / 107 / 186 / 788, 20.6, 395
+//   FP32 MRT     12.5 / 18.7 / 47.5 / 113 / 195 / 828, 21.4, 436
+//   (general,    12.5 / 18.8 / 47.5 / 114 / 195 / 810, 21.4, 428
+//   spills at 4) 10.4 / 18.1 / 44.1 / 110 / 192 / 810, 22.7, 410
+//   FP16S BGK    12.5 / 16.3 / 26.4 / 62.7 / 104 / 415, 17.1, 216
+//                12.4 / 16.3 / 26.3 / 62.7 / 106 / 430, 16.9, 226
+//                 8.4 / 16.5 / 34.9 / 95.3 / 176 / 710, 19.3, 402
+//   FP16S MRT    12.5 / 16.8 / 30.8 / 71.2 / 119 / 474, 19.8, 265
+//                12.5 / 16.9 / 30.8 / 71.1 / 122 / 483, 19.8, 275
+//                 8.4 / 15.3 / 31.0 / 90.0 / 164 / 665, 18.6, 368
+//   FP64 BGK     12.5 / 24.8 / 66.4 / 165 / 291 / 1245, 37.2, 647
+//                12.4 / 24.8 / 65.7 / 166 / 292 / 1250, 37.1, 661
+//                10.4 / 23.3 / 67.8 / 174 / 308 / 1333, 37.0, 711
+// So FP32 and FP16S at 2 cells up to 400,000 padded cells, general FP32 MRT at 2
+// cells always; above, one tile a CTA for FP32 BGK and LES and a persistent grid for
+// the rest.  FP64 at 2 cells in a persistent grid.  FP32S keeps one tile a CTA at 2
+// cells.
 // One block, FP32, FP32S and FP64: 2 warps a CTA, 2 cells a thread.  4 warps took
 // 107 / 390 / 198 us for 103 / 385 / 192 (FP32 BGK 160^3, 242^3, 319 x 205 x 123),
 // 474 for 457 (LES 258^3), 471 for 457 (FP32S 256^3), 428 for 419 (FP64 202^3).
@@ -370,7 +396,11 @@ Shape auto_shape(const flb_lattice* h) {
   const int storage = h->desc.storage;
   if (h->mode >= 0) {
     if (storage == FLB_STORAGE_FP32S) return {4, 0, 2};
-    return {4, 32, storage == FLB_STORAGE_FP64 ? 2 : 4};
+    if (storage == FLB_STORAGE_FP64) return {4, 32, 2};
+    const bool mrt = h->desc.model == FLB_MODEL_MRT;
+    const bool general = storage == FLB_STORAGE_FP32 && mrt && !use_mrt2(h);
+    if (general || h->dstride <= 400000) return {4, 0, 2};
+    return {4, storage == FLB_STORAGE_FP32 && !mrt ? 0 : 32, 4};
   }
   const HostBlock& b = h->blocks[0];
   const long long cells = (long long)b.L.nx * b.L.ny * b.L.nz;

@@ -302,3 +302,38 @@ def test_autotune_leaves_the_winner_ready_to_be_captured(gpu_ok):
     b.step(taken + 2)
     for k in range(a.nblocks):
         assert np.array_equal(a.download_pops(block=k), b.download_pops(block=k))
+
+
+GENERAL = [0, 1.1, 1.3, 0, 1.25, 0, 1.25, 0, 1.25, 1, 1.4, 1, 1.4, 1, 1, 1, 1.5, 1.5, 1.5]
+
+
+@pytest.mark.parametrize("storage,kw,count,want", [
+    ("fp32", {}, 1, (4, 0, 2)), ("fp32", {}, 2, (4, 0, 4)),
+    ("fp32", {"model": "les"}, 2, (4, 0, 4)),
+    ("fp32", {"model": "mrt"}, 1, (4, 0, 2)), ("fp32", {"model": "mrt"}, 2, (4, 32, 4)),
+    ("fp32", {"model": "mrt", "mrt_rate": GENERAL}, 2, (4, 0, 2)),
+    ("fp16s", {}, 1, (4, 0, 2)), ("fp16s", {"model": "mrt"}, 2, (4, 32, 4)),
+    ("fp16s", {"model": "mrt", "mrt_rate": GENERAL}, 2, (4, 32, 4)),
+    ("fp64", {}, 1, (4, 32, 2)), ("fp32s", {"model": "mrt"}, 2, (4, 0, 2)),
+])
+def test_default_shapes_of_many_blocks(gpu_ok, storage, kw, count, want):
+    """One and two cavities of 60^3 stored cells, on both sides of the rule's
+    400,000, against another shape, bit for bit."""
+    flags = F.cavity_flags(58)
+    u = np.zeros((flags.size, 3))
+    u[flags == 8, 0] = 0.1
+    out = []
+    for chosen in (None, (8, 0, 2)):
+        lat = F.Lattice.blocks([(60, 60, 60, 0, 0, 0)] * count, 0.55, mode="independent",
+                               storage=storage, **kw)
+        for k in range(count):
+            lat.upload_flags(flags, block=k)
+            lat.upload_field("u", u, block=k)
+        if chosen:
+            lat.set_launch(*chosen)
+        else:
+            assert lat.get_launch() == want
+        lat.step(6)
+        out.append([lat.download_pops(block=k) for k in range(count)])
+        lat.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
