@@ -2164,7 +2164,8 @@ static int adjoint_backward_t(flb_lattice* h, double* dJ_dalpha, double* dJ_dtau
   FLB_CUDA(cudaGetLastError());
   int cur = 0;
   const long long chunks = (long long)(b.L.pitch / V) * b.L.ny * b.L.nz;
-  const dim3 block(32 * std::max(h->tile_y, 4));
+  // 4 warps unless the caller chose (the sweep wants them where the step's default is 2)
+  const dim3 block(32 * (h->shape_chosen ? h->tile_y : 4));
   const dim3 grid(unsigned((chunks + block.x - 1) / block.x));
   const size_t npart = 2 * size_t(grid.x);
   if (h->adj_gpart_n < npart) {
