@@ -42,6 +42,8 @@ int fail(int code, const char* fmt, ...) {
   std::vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
   g_err = buf;
+  // reported here: the next call's check of its launches starts clean
+  if (code == FLB_ERR_CUDA || code == FLB_ERR_OOM) cudaGetLastError();
   return code;
 }
 

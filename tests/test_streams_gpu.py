@@ -114,3 +114,21 @@ def test_every_step_kernel_keeps_its_order(gpu_ok, make):
         out.append([lat.download_pops(block=b) for b in range(lat.nblocks)])
         lat.close()
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def test_a_reported_error_does_not_fail_the_next_call(gpu_ok):
+    """A download on a stream that is being captured is an error, once."""
+    import torch
+    from cuda.bindings import runtime as rt
+    lat = F.cavity(20)
+    lat.step(3)
+    want = lat.download_pops()
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    mode = rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal
+    assert rt.cudaStreamBeginCapture(stream.cuda_stream, mode)[0] == 0
+    with pytest.raises(F.FlbError):
+        lat.download_pops(stream=stream)
+    rt.cudaStreamEndCapture(stream.cuda_stream)
+    rt.cudaGetLastError()
+    assert np.array_equal(lat.download_pops(stream=stream), want)
