@@ -8,6 +8,8 @@ tau and the lid speed.  Tolerances are stated per test.  The per-cell bar is
 storage of f itself carries a trajectory error of ~1e-5 that leaves cells with
 small gradients above 1e-4, so it is held to 1e-3.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -193,3 +195,36 @@ def test_objective_and_conservation_sums_are_deterministic(gpu_ok, storage):
     assert len(js) == 1, js
     sums = [lat.conservation(key=2) for _ in range(5)]
     assert all(np.array_equal(s, sums[0]) for s in sums)
+
+
+def test_gradient_takes_no_memory_beyond_its_own(gpu_ok):
+    """dJ/dalpha leaves the device through the sweep's own arrays: the pair does not
+    grow the handle's staging buffer (8 bytes a cell), which no release frees."""
+    b = F.Lattice(22, 22, 22, 0.56, storage="fp32s", model="brinkman")
+    b.upload_flags(F.cavity_flags(20))
+    before = b.memory_bytes()
+    b.adjoint_forward(6, 3)
+    b.adjoint_backward()
+    assert b.memory_bytes() == before
+
+
+def test_gradient_array_is_left_alone_by_a_call_that_fails(gpu_ok):
+    """A sweep whose results cannot be copied (its stream is being captured) is an
+    error, and the caller's array keeps what it held; the next call fills it."""
+    import torch
+    from cuda.bindings import runtime as rt
+    lat = brinkman_cavity(20, 0.56, 0.1, O.porosity(20, 5), "fp32s")
+    stream = torch.cuda.Stream()
+    lat.adjoint_forward(6, 3, stream=stream)
+    want = lat.adjoint_backward(stream=stream)[0]
+    got = np.full(lat.N, 7.0)
+    call = F._capi.load().flb_adjoint_backward
+    raw = ctypes.c_void_p(stream.cuda_stream)
+    mode = rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal
+    assert rt.cudaStreamBeginCapture(stream.cuda_stream, mode)[0] == 0
+    rc = call(lat._h, got.ctypes.data_as(ctypes.c_void_p), None, None, raw)
+    rt.cudaStreamEndCapture(stream.cuda_stream)
+    rt.cudaGetLastError()
+    assert rc == -2 and np.all(got == 7.0)        # FLB_ERR_CUDA
+    assert call(lat._h, got.ctypes.data_as(ctypes.c_void_p), None, None, raw) == 0
+    assert np.array_equal(got, want)
