@@ -96,6 +96,7 @@ SIGNATURES = {
     "flb_device_status": [_P, _P],
     "flb_test_withhold_tile": [_P, ctypes.c_longlong],
     "flb_test_wide_offsets": [_P, _I],
+    "flb_test_quotient": [ctypes.c_longlong, _P, _P, _P],
     "flb_set_rounding": [_P, _I],
     "flb_snapshot_bytes": [_P, ctypes.POINTER(ctypes.c_size_t)],
     "flb_snapshot_save": [_P, _P, ctypes.c_size_t, _P],

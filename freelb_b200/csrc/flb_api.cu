@@ -1696,6 +1696,24 @@ int flb_test_withhold_tile(flb_lattice* h, long long tile) {
   return FLB_OK;
 }
 
+int flb_test_quotient(long long n, const float* m, const float* den, float* q) {
+  if (n < 1 || n > (1LL << 28) || !m || !den || !q)
+    return fail(FLB_ERR_INVALID, "flb_test_quotient: bad arguments");
+  const size_t bytes = size_t(n) * sizeof(float);
+  float* d = nullptr;
+  FLB_CUDA(cudaMalloc((void**)&d, 3 * bytes));
+  cudaError_t e = cudaMemcpy(d, m, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + n, den, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_test_quotient<<<unsigned((n + 255) / 256), 256>>>(n, d, d + n, d + 2 * n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(q, d + 2 * n, bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) return fail(FLB_ERR_CUDA, "flb_test_quotient: %s", cudaGetErrorString(e));
+  return FLB_OK;
+}
+
 int flb_test_wide_offsets(flb_lattice* h, int on) {
   if (!h) return fail(FLB_ERR_INVALID, "null handle");
   if (on && h->shape_chosen && h->ctas_per_sm < 0)

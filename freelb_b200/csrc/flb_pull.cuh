@@ -834,7 +834,8 @@ __device__ __forceinline__ void les_deviation2(const StepParams& p, float2 (&H)[
 
 // ---------------------------------------------------------------------------
 // FP32S storage (dev32): d_i = f_i - rho0 w_i in FP32, collided as stored, the
-// FP16S deviation form at full FP32 width with IEEE divisions.
+// FP16S deviation form at full FP32 width; u by IEEE divisions (dev_moments), or
+// by the refined quotient of the two-wide form below.
 
 // delta = sum d (= rho - rho0), rho, den = rho + alpha/2 and u = sum c d / den
 // (the weights carry no momentum, so sum c d = sum c f); alpha = 0 gives
@@ -932,12 +933,17 @@ __device__ __forceinline__ void collide_dev32(const StepParams& p, int op, float
 // FP32S in the pair form: two cells per two-wide instruction, every operation
 // explicit, so a cell's result does not depend on the cell it is paired with.
 // u = m / den comes from one reciprocal and a residual step (Markstein 1990:
-// q = m r, q + r (m - den q)), which rounds as the IEEE division does but for
-// rare last-bit cases, for three components at the price of one.  130^3 Brinkman
-// step 74.6 -> 65.6 us (53 us at 6.65 TB/s); MRT and LES keep the scalar form.
+// q = m r, q + r (m - den q)), for three components at the price of one.  It is the
+// rounded quotient unless m / den lies within 2^-22 ulp of a tie; of 6e8 random pairs
+// (den 1e-3 to 1e6, |m / den| 1e-20 to 1) none differed from the IEEE division.  130^3
+// Brinkman step 74.6 -> 65.6 us (54 us at 6.55 TB/s); MRT and LES keep the scalar form.
 struct DevMoments {
   float2 delta, rho, den, ux, uy, uz;
 };
+__device__ __forceinline__ float2 refined_reciprocal(float2 den) {
+  const float2 r = make_float2(__fdividef(1.0f, den.x), __fdividef(1.0f, den.y));
+  return fma2(r, fma2(mul2(p2(-1.0f), den), r, p2(1.0f)), r);
+}
 __device__ __forceinline__ float2 refined_quotient(float2 m, float2 den, float2 r) {
   const float2 q = mul2(m, r);
   return fma2(fma2(mul2(p2(-1.0f), den), q, m), r, q);
@@ -956,8 +962,7 @@ __device__ __forceinline__ DevMoments dev_moments2(const float2 (&d)[Q], float r
                  add2(sp[7], sp[8]));
   m.rho = add2(p2(rho0), m.delta);
   m.den = fma2(p2(0.5f), alpha, m.rho);
-  float2 r = make_float2(__fdividef(1.0f, m.den.x), __fdividef(1.0f, m.den.y));
-  r = fma2(r, fma2(mul2(p2(-1.0f), m.den), r, p2(1.0f)), r);
+  const float2 r = refined_reciprocal(m.den);
   m.ux = refined_quotient(add2(add2(add2(df[0], df[3]), add2(df[4], df[6])), df[7]), m.den, r);
   m.uy = refined_quotient(add2(add2(add2(df[1], df[3]), sub2(df[5], df[6])), df[8]), m.den, r);
   m.uz = refined_quotient(sub2(add2(add2(df[2], df[4]), sub2(df[5], df[7])), df[8]), m.den, r);
@@ -1006,6 +1011,14 @@ __device__ __forceinline__ void brinkman_dev2(float2 (&d)[Q], float omega, float
     d[i] = fma2(c1, d[i], mul2(w, add2(ge, go)));
     d[i + 1] = fma2(c1, d[i + 1], mul2(w, sub2(ge, go)));
   }
+}
+
+// q = m / den as dev_moments2 forms it (flb_test_quotient).
+static __global__ void k_test_quotient(long long n, const float* m, const float* den, float* q) {
+  const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const float2 d = p2(den[k]);
+  q[k] = refined_quotient(p2(m[k]), d, refined_reciprocal(d)).x;
 }
 
 // Two FP32S cells (ca, ca + 1) by their ops, in place.

@@ -387,6 +387,10 @@ FLB_API int flb_test_withhold_tile(flb_lattice* lat, long long tile);
  * that path can be checked on a small lattice. */
 FLB_API int flb_test_wide_offsets(flb_lattice* lat, int on);
 
+/* Test hook: q[k] = m[k] / den[k] for n host values, in the arithmetic by which the
+ * FP32S BGK and Brinkman step forms a velocity. */
+FLB_API int flb_test_quotient(long long n, const float* m, const float* den, float* q);
+
 /* Autotuner: times every candidate launch shape for `trial_steps` steps on
  * `stream` (CUDA events) and keeps the fastest.  The trial steps are real
  * time steps: the lattice advances by *steps_taken.  best_ms = time per step

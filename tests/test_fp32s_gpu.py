@@ -9,6 +9,8 @@ the single-block run bit for bit on fluid cells and the transfers convert the
 deviations (the post-stream bounce-back managers are covered in
 test_boundary_gpu.py, the adjoint in test_adjoint_gpu.py).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -152,3 +154,27 @@ def test_fp32s_graph_and_autotune(gpu_ok):
     a.step(6, graph=True)
     b.step(6)
     assert np.array_equal(a.download_pops(), b.download_pops())
+
+
+def quotient(m, den):
+    q = np.empty_like(m)
+    F._capi.call("flb_test_quotient", m.size, *(a.ctypes.data_as(ctypes.c_void_p)
+                                                for a in (m, den, q)))
+    return q
+
+
+@pytest.mark.parametrize("lo,hi", [(0.9, 1.1), (0.5, 2.0), (1e-3, 1e6)])
+def test_refined_quotient_rounds_as_the_division(gpu_ok, lo, hi):
+    """u = m / den of the two-wide BGK and Brinkman step, den = rho + alpha / 2.  The
+    refined reciprocal r is within an ulp, so m r is within two ulps, its residual
+    is exact, and the correction r (m - den q) carries an error of 2 x 2^-23 ulp: the
+    result is the rounded quotient unless m / den lies that near a tie, at most one
+    pair in 2^20, and then the neighbouring value."""
+    n = 1 << 22
+    rng = np.random.default_rng(int(hi))
+    den = np.exp(rng.uniform(np.log(lo), np.log(hi), n)).astype(np.float32)
+    ratio = np.exp(rng.uniform(np.log(1e-20), 0, n)) * rng.choice([-1.0, 1.0], n)
+    m = (den * ratio).astype(np.float32)
+    m[:4] = [0.0, den[1], -den[2], np.nextafter(den[3], np.float32(0))]
+    off = np.abs(quotient(m, den).view(np.int32).astype(np.int64) - (m / den).view(np.int32))
+    assert off.max() <= 1 and np.count_nonzero(off) <= n * 2.0 ** -20
