@@ -201,8 +201,8 @@ int grid_1d(long long n) {
 // Kernels that read a block in chunks of ReadWidth cells: one chunk a thread up
 // to 8 CTAs per SM, then a grid stride (few partial results to add up).
 template <typename S>
-int read_grid(const HostBlock& b) {
-  return std::min(grid_1d(b.padded() / ReadWidth<S>::V), 148 * 8);
+int read_grid(const flb_lattice* h, const HostBlock& b) {
+  return std::min(grid_1d(b.padded() / ReadWidth<S>::V), h->sm_count * 8);
 }
 
 // k_halo_pull32: enough 256-thread CTAs for one batch of HALO_BATCH records
@@ -333,11 +333,17 @@ struct Shape {
 };
 
 // Lattices that k_pull steps in its SMALL form: up to 300,000 padded cells, 64^3
-// and the like.  Us a step in a graph of two, without / with it, at 32 / 48 / 64 /
-// 72 stored cells a side: FP32 BGK 5.13 / 7.16 / 9.42 / 12.2 and 4.12 / 6.16 /
-// 9.25 / 12.3, LES 4.38 / 7.19 / 10.3 / 12.8 and 5.13 / 6.16 / 10.3 / 13.3 (12^3:
-// 5.14 and 4.13), FP16S BGK 6.16 / 6.34 / 9.71 / 11.3 and 4.12 / 5.15 / 7.21 / 9.61,
-// FP64 5.15 / 8.21 / 15.4 / 23.7 and 5.16 / 7.20 / 15.4 / 23.6.
+// and the like.  Us a step without / with it at 24 / 32 / 48 / 64 stored cells a side,
+// launched one by one (in a graph of two, to its microsecond steps):
+//   FP32 BGK   4.77 / 4.98 / 6.51 / 8.52 and 3.88 / 4.88 / 5.24 / 8.46
+//              (5.1 / 5.1 / 7.2 / 9.4 and 4.1 / 4.1 / 6.2 / 9.2)
+//   FP32 LES   4.68 / 5.37 / 6.54 / 9.32 and 4.12 / 5.35 / 5.72 / 9.14
+//              (5.1 / 5.1 / 7.2 / 10.3 and 5.1 / 5.1 / 6.2 / 10.3)
+//   FP16S BGK  5.67 / 5.49 / 6.16 / 8.73 and 3.49 / 3.88 / 4.51 / 6.48
+//   FP64 BGK   5.00 / 5.89 / 6.93 / 14.4 and 5.03 / 5.89 / 6.33 / 14.4
+//   FP32S MRT  5.30 / 6.69 / 7.45 / 11.3 and 4.38 / 6.15 / 6.62 / 10.7
+// At 72^3 (413,000) FP32 BGK and LES are level or lose in a graph (12.2 / 12.8 and 12.3
+// / 13.3).
 bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 
 // Shape of a handle's steps until flb_set_launch or flb_autotune chooses one.
@@ -1857,7 +1863,7 @@ int flb_compute_rhou(flb_lattice* h, uint8_t key, void* stream) {
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     return for_blocks(h, [&](const HostBlock& b) {
-      k_rhou_pull<S, R, ReadWidth<S>::V><<<read_grid<S>(b), 256, 0, st>>>(
+      k_rhou_pull<S, R, ReadWidth<S>::V><<<read_grid<S>(h, b), 256, 0, st>>>(
           geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->flags, key,
           static_cast<R*>(h->rho), static_cast<R*>(h->vel), h->sp);
       return FLB_OK;
@@ -1875,7 +1881,7 @@ int flb_reduce_conservation(flb_lattice* h, uint8_t key, double out[4], void* st
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     return for_blocks(h, [&](const HostBlock& b) {
-      const int grid = read_grid<S>(b);
+      const int grid = read_grid<S>(h, b);
       k_conservation_pull<S, R, ReadWidth<S>::V><<<grid, 256, 0, st>>>(
           geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->flags, key, h->red,
           h->sp);
@@ -1901,7 +1907,7 @@ int flb_tolerance_u(flb_lattice* h, uint8_t key, double* max_du, void* stream) {
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     return for_blocks(h, [&](const HostBlock& b) {
-      k_tolerance_pull<S, R, ReadWidth<S>::V><<<read_grid<S>(b), 256, 0, st>>>(
+      k_tolerance_pull<S, R, ReadWidth<S>::V><<<read_grid<S>(h, b), 256, 0, st>>>(
           geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->flags, key, h->uprev,
           acc, h->sp);
       return FLB_OK;
@@ -2055,7 +2061,7 @@ int flb_objective_u2(flb_lattice* h, double* J, void* stream) {
     using S = std::remove_pointer_t<decltype(sp)>;
     using R = std::remove_pointer_t<decltype(rp)>;
     if constexpr (!std::is_same<S, __half>::value) {
-      const int grid = read_grid<S>(b);
+      const int grid = read_grid<S>(h, b);
       k_objective<S, R, ReadWidth<S>::V><<<grid, 256, 0, st>>>(
           geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->sp, (R*)nullptr,
           (double*)nullptr, h->red, false);
@@ -2195,7 +2201,7 @@ static int adjoint_backward_t(flb_lattice* h, double* dJ_dalpha, double* dJ_dtau
     h->adj_seg.push_back(p);
   }
   // seed lambda_T = dJ/dR_T and the direct dJ/dalpha term (the J partials are unused)
-  k_objective<S, R, ReadWidth<S>::V><<<read_grid<S>(b), 256, 0, st>>>(
+  k_objective<S, R, ReadWidth<S>::V><<<read_grid<S>(h, b), 256, 0, st>>>(
       geom_of(b), h->dstride, static_cast<const S*>(h->pops[h->cur]), h->sp,
       static_cast<R*>(h->adj_lam[0]), h->alpha ? h->adj_galpha : nullptr, h->red, true);
   FLB_CUDA(cudaGetLastError());

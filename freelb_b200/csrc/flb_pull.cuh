@@ -1527,7 +1527,7 @@ __device__ __forceinline__ void gather_stored(const S* pops, long long dstride, 
 // walk chunks of V cells with the step kernels' vector gather and 32-bit index
 // arithmetic.  202^3 FP32, us: fields 147 (260 with a scalar gather, its wrap
 // rule and 64-bit divisions a cell), sums 133 (350), check 173 (1090); the bytes
-// they cannot do without take 113, 96 and 157 at 6.65 TB/s.
+// they cannot do without take 115, 98 and 159 at 6.55 TB/s.
 template <typename S>
 struct ReadWidth {
   static constexpr int V = std::is_same<S, __half>::value ? 4 : 2;  // cells per thread
