@@ -364,36 +364,37 @@ bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 // sides meet between 96^3 and 128^3.  Where the rows do not suit the bulk
 // copies, BGK and LES change to 4 cells a thread there and MRT (whose 4-cell
 // form spills) at 10 M cells (between 192^3 and 256^3).
-// Many blocks, 4 warps a CTA.  Us a step of persistent grids (32 CTAs an SM) at the
+// Many blocks, 4 warps a CTA.  Us a step of a persistent grid (32 CTAs an SM) at the
 // larger number of cells a thread / one tile a CTA, the same / one tile a CTA at 2
-// cells (FP64: 1), for cavities of 48 / 64 / 96 / 128 / 160 / 256 cells a side in uneven
-// blocks (0.13 / 0.31 / 0.98 / 2.4 / 4.6 / 18.8 M padded cells), then 4 (0.51 M) and 16
-// (11.6 M) independent ones:
-//   FP32 BGK     12.2 / 16.8 / 42.5 / 96.7 / 161 / 674, 18.7, 342
-//                12.1 / 16.6 / 39.4 / 89.0 / 150 / 626, 18.5, 318
-//                 8.4 / 14.6 / 39.7 / 101 / 174 / 742, 18.6, 366
-//   FP32 LES     12.5 / 18.0 / 43.6 / 104 / 177 / 756, 20.4, 391
-//                12.4 / 17.5 / 43.1 / 101 / 172 / 705, 19.8, 372
-//                 8.7 / 16.5 / 42.5 / 105 / 180 / 768, 20.6, 383
-//   FP32 MRT     12.5 / 17.8 / 41.2 / 94.5 / 159 / 667, 19.4, 341
-//   (two-rate)   12.5 / 17.4 / 41.2 / 94.8 / 162 / 666, 19.3, 344
-//                10.1 / 16.6 / 43.2 / 107 / 186 / 788, 20.6, 395
-//   FP32 MRT     12.5 / 18.7 / 47.5 / 113 / 195 / 828, 21.4, 436
-//   (general,    12.5 / 18.8 / 47.5 / 114 / 195 / 810, 21.4, 428
-//   spills at 4) 10.4 / 18.1 / 44.1 / 110 / 192 / 810, 22.7, 410
-//   FP16S BGK    12.5 / 16.3 / 26.4 / 62.7 / 104 / 415, 17.1, 216
-//                12.4 / 16.3 / 26.3 / 62.7 / 106 / 430, 16.9, 226
-//                 8.4 / 16.5 / 34.9 / 95.3 / 176 / 710, 19.3, 402
-//   FP16S MRT    12.5 / 16.8 / 30.8 / 71.2 / 119 / 474, 19.8, 265
-//                12.5 / 16.9 / 30.8 / 71.1 / 122 / 483, 19.8, 275
-//                 8.4 / 15.3 / 31.0 / 90.0 / 164 / 665, 18.6, 368
-//   FP64 BGK     12.5 / 24.8 / 66.4 / 165 / 291 / 1245, 37.2, 647
-//                12.4 / 24.8 / 65.7 / 166 / 292 / 1250, 37.1, 661
-//                10.4 / 23.3 / 67.8 / 174 / 308 / 1333, 37.0, 711
-// So FP32 and FP16S at 2 cells up to 400,000 padded cells, general FP32 MRT at 2
-// cells always; above, one tile a CTA for FP32 BGK and LES and a persistent grid for
-// the rest.  FP64 at 2 cells in a persistent grid.  FP32S keeps one tile a CTA at 2
-// cells.
+// cells (FP64: 1), for cavities of 48 / 64 / 80 / 96 / 128 / 160 / 224 cells a side in
+// uneven blocks (0.13 / 0.31 / 0.62 / 0.98 / 2.4 / 4.6 / 12.5 M padded cells), then 4
+// (0.51 M) and 16 (9.3 M) independent ones; median of five rounds of the shapes in
+// turn, on a flow of its own in every cell (the first steps from rest are slower: the
+// divisions meet denormals):
+//   FP32 BGK     12.3 / 16.5 / 29.2 / 39.0 / 87.7 / 146 / 398, 18.3, 250
+//                12.2 / 16.4 / 29.2 / 39.0 / 87.7 / 149 / 401, 18.3, 254
+//                 8.3 / 14.4 / 30.2 / 39.2 / 100 / 173 / 477, 18.5, 300
+//   FP32 LES     12.4 / 16.6 / 30.9 / 41.1 / 95.5 / 162 / 440, 18.7, 283
+//                12.4 / 16.6 / 31.0 / 41.1 / 95.6 / 164 / 435, 18.6, 281
+//                 8.8 / 16.4 / 31.1 / 41.1 / 103 / 180 / 492, 18.8, 312
+//   FP32 MRT     12.4 / 17.5 / 30.7 / 41.1 / 94.2 / 159 / 429, 19.5, 279
+//   (two-rate)   12.4 / 17.5 / 30.6 / 41.1 / 94.4 / 161 / 431, 19.2, 279
+//                10.3 / 16.5 / 32.9 / 43.1 / 107 / 186 / 509, 20.6, 325
+//   FP32 MRT     12.4 / 18.1 / 32.2 / 43.2 / 101 / 175 / 477, 20.3, 308
+//   (general)    12.4 / 18.1 / 32.3 / 43.2 / 101 / 176 / 475, 20.3, 305
+//                10.2 / 16.5 / 32.1 / 41.2 / 105 / 184 / 504, 20.6, 320
+//   FP16S BGK    12.4 / 16.5 / 24.3 / 26.2 / 62.8 / 104 / 272, 16.9, 179
+//                12.3 / 16.4 / 24.2 / 26.1 / 63.0 / 106 / 282, 17.0, 185
+//                 8.3 / 16.5 / 26.7 / 34.4 / 95.4 / 176 / 470, 19.2, 327
+//   FP16S MRT    12.4 / 17.0 / 26.9 / 30.7 / 71.4 / 119 / 310, 19.6, 218
+//                12.4 / 16.9 / 26.8 / 30.6 / 71.5 / 122 / 319, 19.8, 224
+//                 8.3 / 15.3 / 24.8 / 30.8 / 90.1 / 164 / 439, 18.5, 299
+//   FP64 BGK     at 48 / 64 / 96 / 160 and 4: 12.4 / 24.8 / 65.2 / 283, 36.9
+//                                             12.4 / 24.8 / 65.2 / 290, 36.9
+//                                             10.3 / 23.3 / 67.5 / 306, 36.9
+// So a persistent grid at 4 cells (FP64: 2), and one tile a CTA at 2 cells (FP64: 1)
+// up to 400,000 padded cells, in general FP32 MRT, which spills at 4 cells, up to
+// 1.2 M.  FP32S keeps one tile a CTA at 2 cells.
 // One block, FP32, FP32S and FP64: 2 warps a CTA, 2 cells a thread.  4 warps took
 // 107 / 390 / 198 us for 103 / 385 / 192 (FP32 BGK 160^3, 242^3, 319 x 205 x 123),
 // 474 for 457 (LES 258^3), 471 for 457 (FP32S 256^3), 428 for 419 (FP64 202^3).
@@ -407,11 +408,12 @@ Shape auto_shape(const flb_lattice* h) {
   const int storage = h->desc.storage;
   if (h->mode >= 0) {
     if (storage == FLB_STORAGE_FP32S) return {4, 0, 2};
-    if (storage == FLB_STORAGE_FP64) return {4, 32, 2};
-    const bool mrt = h->desc.model == FLB_MODEL_MRT;
-    const bool general = storage == FLB_STORAGE_FP32 && mrt && !use_mrt2(h);
-    if (general || h->dstride <= 400000) return {4, 0, 2};
-    return {4, storage == FLB_STORAGE_FP32 && !mrt ? 0 : 32, 4};
+    if (storage == FLB_STORAGE_FP64)
+      return h->dstride <= 400000 ? Shape{4, 0, 1} : Shape{4, 32, 2};
+    const bool general = storage == FLB_STORAGE_FP32 && h->desc.model == FLB_MODEL_MRT &&
+                         !use_mrt2(h);
+    if (h->dstride <= (general ? 1200000 : 400000)) return {4, 0, 2};
+    return {4, 32, 4};
   }
   const HostBlock& b = h->blocks[0];
   const long long cells = (long long)b.L.nx * b.L.ny * b.L.nz;

@@ -323,8 +323,8 @@ FLB_API int flb_download_field_block(flb_lattice* lat, int block, int field, voi
  * warps run 2-cell chunks).  Its waits are bounded (flb_set_wait_limit).
  * Without a call the library picks a shape by storage, model and size
  * (flb_get_launch tells which): small FP16S lattices 2 cells per thread, large
- * ones the bulk-copy kernel where the rows suit it, multi-block handles a
- * persistent grid, and otherwise one CTA of 2 or 4 warps per tile. */
+ * ones the bulk-copy kernel where the rows suit it, larger multi-block handles
+ * a persistent grid, and otherwise one CTA of 2 or 4 warps per tile. */
 FLB_API int flb_set_launch(flb_lattice* lat, int tile_y, int ctas_per_sm, int cells_per_thread);
 FLB_API int flb_get_launch(const flb_lattice* lat, int* tile_y, int* ctas_per_sm,
                            int* cells_per_thread);

@@ -308,17 +308,18 @@ GENERAL = [0, 1.1, 1.3, 0, 1.25, 0, 1.25, 0, 1.25, 1, 1.4, 1, 1.4, 1, 1, 1, 1.5,
 
 
 @pytest.mark.parametrize("storage,kw,count,want", [
-    ("fp32", {}, 1, (4, 0, 2)), ("fp32", {}, 2, (4, 0, 4)),
-    ("fp32", {"model": "les"}, 2, (4, 0, 4)),
+    ("fp32", {}, 1, (4, 0, 2)), ("fp32", {}, 2, (4, 32, 4)),
+    ("fp32", {"model": "les"}, 2, (4, 32, 4)),
     ("fp32", {"model": "mrt"}, 1, (4, 0, 2)), ("fp32", {"model": "mrt"}, 2, (4, 32, 4)),
-    ("fp32", {"model": "mrt", "mrt_rate": GENERAL}, 2, (4, 0, 2)),
+    ("fp32", {"model": "mrt", "mrt_rate": GENERAL}, 5, (4, 0, 2)),
+    ("fp32", {"model": "mrt", "mrt_rate": GENERAL}, 6, (4, 32, 4)),
     ("fp16s", {}, 1, (4, 0, 2)), ("fp16s", {"model": "mrt"}, 2, (4, 32, 4)),
     ("fp16s", {"model": "mrt", "mrt_rate": GENERAL}, 2, (4, 32, 4)),
-    ("fp64", {}, 1, (4, 32, 2)), ("fp32s", {"model": "mrt"}, 2, (4, 0, 2)),
+    ("fp64", {}, 1, (4, 0, 1)), ("fp64", {}, 2, (4, 32, 2)), ("fp32s", {"model": "mrt"}, 2, (4, 0, 2)),
 ])
 def test_default_shapes_of_many_blocks(gpu_ok, storage, kw, count, want):
-    """One and two cavities of 60^3 stored cells, on both sides of the rule's
-    400,000, against another shape, bit for bit."""
+    """Cavities of 60^3 stored cells (216,000 each) on both sides of the rule's
+    lines, against another shape, bit for bit."""
     flags = F.cavity_flags(58)
     u = np.zeros((flags.size, 3))
     u[flags == 8, 0] = 0.1
