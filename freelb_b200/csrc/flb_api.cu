@@ -360,10 +360,14 @@ bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 //              bulk copy (-2)    10.3 / 14.4 / 26.7 / 48 / 128 / 296 / 534
 // Small lattices are bound by one thread's chain of work, so fewer cells a
 // thread; large FP16S ones by the loads in flight, which the bulk copies take
-// off the registers.  The line between them lies at 1.2 M cells (106^3): the
-// sides meet between 96^3 and 128^3.  Where the rows do not suit the bulk
-// copies, BGK and LES change to 4 cells a thread there and MRT (whose 4-cell
-// form spills) at 10 M cells (between 192^3 and 256^3).
+// off the registers.  The line between them lies at 1.2 M cells (106^3), for BGK at
+// 1.05 M (2 / 4 cells a thread: 96^3 18.4 / 19.0 us, 100^3 20.7 / 21.3, 102^3 22.8 / 22.2,
+// 104^3 24.7 / 23.7, 106^3 27.5 / 25.1; LES 104^3 27.1 / 28.2, 106^3 29.8 / 28.8).  Past it,
+// rows that suit the bulk copies take them (bulk_copy_rows); the others 4 cells a
+// thread, but MRT, whose 4-cell form spills, 2 below 10 M cells unless the last
+// chunk of a row holds 2 or 3 cells.  MRT at 2 / 4 cells: 120^3 44.2 / 48.5 us, 128^3
+// 52.2 / 55.7, 192^3 156 / 165, 293 x 200 x 130 192 / 196; 127^3 56.1 / 54.0, 158^3 96.2 /
+// 88.7, 202^3 190 / 178, 319 x 200 x 130 198 / 181, 50 x 500 x 300 204 / 172.
 // Many blocks, 4 warps a CTA.  Us a step of a persistent grid (32 CTAs an SM) at the
 // larger number of cells a thread / one tile a CTA, the same / one tile a CTA at 2
 // cells (FP64: 1), for cavities of 48 / 64 / 80 / 96 / 128 / 160 / 224 cells a side in
@@ -404,6 +408,7 @@ bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 // 182^3, 202^3, 130 x 300 x 200 and 66 x 400 x 350; on aligned rows (160^3: 108 for
 // 103; 242^3: 423 for 385) and smaller lattices (152^3: 94 for 88) it loses, and MRT
 // and LES, which spill in it, lose nearly everywhere.
+bool bulk_copy_rows(const flb_lattice* h, long long cells);
 Shape auto_shape(const flb_lattice* h) {
   const int storage = h->desc.storage;
   if (h->mode >= 0) {
@@ -417,15 +422,55 @@ Shape auto_shape(const flb_lattice* h) {
   }
   const HostBlock& b = h->blocks[0];
   const long long cells = (long long)b.L.nx * b.L.ny * b.L.nz;
-  const bool large = cells >= 1200000;
+  const bool large = cells >= (h->desc.model == FLB_MODEL_BGK ? 1050000 : 1200000);
   if (storage != FLB_STORAGE_FP16S) {
     if (small_lattice(b)) return {4, 0, 2};
     const bool wide = storage == FLB_STORAGE_FP32 && h->desc.model == FLB_MODEL_BGK &&
                       b.L.pitch % 32 != 0 && cells >= 4500000;
     return {2, 0, wide ? 4 : 2};
   }
-  if (large && tma_supported(h)) return {4, -2, 4};
-  return {4, 0, (h->desc.model == FLB_MODEL_MRT ? cells >= 10000000 : large) ? 4 : 2};
+  if (bulk_copy_rows(h, cells)) return {4, -2, 4};
+  const bool mrt = h->desc.model == FLB_MODEL_MRT;
+  return {4, 0, large && (!mrt || cells >= 10000000 || b.L.nx % 4 >= 2) ? 4 : 2};
+}
+
+// FP16S lattices whose default is the bulk-copy kernel, by the rows.  Its warps take
+// 64 cells of a tile of 960, and a warp with a row end takes longer.  Where the
+// tiles of a CTA (every sm_count-th) meet the row ends at the same warps each time,
+// the stages wait for those; and row padding that no chunk of 2 covers leaves
+// sectors written in part.  Us a step, bulk copies / the better of 2 and 4 cells a
+// thread, BGK, LES, MRT:
+//   no padding    112^3 32.4 34.6 35.0 / 32.3 35.7 36.4; 128^3 43.5 48.2 49.3 / 43.8 49.7
+//                 52.2; 152^3 61.8 66.4 68.0 / 68.8 79.4 82.1; 104 x 300^2 150 168 172 /
+//                 171 189 213; 88 x 130^2 34.9 37.7 39.0 / 31.1 35.8 38.5
+//     same warps  120^3 44.6 47.8 48.3 / 39.0 43.4 44.2; 240^2 x 120 125 136 139 / 123 139
+//                 152; in half warps 192^3 114 128 132 / 126 147 156, 160 x 164 x 213 102
+//                 113 117 / 104 121 126
+//   one cell      135^3 49.3 56.3 61.3 / 50.8 56.4 65.6; 143^3 56.0 67.8 74.1 / 57.6 64.3
+//                 75.4; 151^3 63.1 73.0 78.4 / 67.3 74.9 88.1; 303 x 200 x 130 121 135 143 /
+//                 136 150 175; 111^3 32.9 37.0 40.7 / 28.9 33.5 38.0
+//     same warps  127^3 49.7 58.6 62.3 / 42.1 46.7 54.0; 319 x 330 x 250 428 509 587 / 431
+//                 474 552
+//   two           126^3 48.6 51.0 52.0 / 41.8 45.1 50.1; 150^3 74.5 76.1 76.0 / 65.8 70.0 79.2;
+//                 182^3 112 112 112 / 108 116 133; 206^3 152 157 158 / 153 162 186; 302 x 200
+//                 x 130 130 136 137 / 133 144 162
+//     same warps  158^3 85.7 89.9 92.4 / 73.6 78.1 88.7; 190^3 126 132 134 / 121 127 145
+//   more          293 x 200 x 130 131 140 147 / 149 169 192; 300 x 200 x 130 130 136 136 / 145
+//                 160 174; 109^3 34.9 38.3 41.7 / 31.5 35.4 38.7; 133 x 376 x 201 195 208 227 /
+//                 193 224 276
+//     same warps  317 x 200 x 130 151 173 198 / 148 169 199; 244 x 94 x 378 157 169 174 / 175
+//                 201 203; 306 x 177 x 209 193 208 215 / 202 216 242; an odd number of
+//                 cells: 245 x 155 x 92 80.2 95.3 103 / 77.9 88.1 92.8; 241 x 360 x 129 239
+//                 286 313 / 234 268 291; 313 x 205 x 123 145 168 192 / 148 171 196
+bool bulk_copy_rows(const flb_lattice* h, long long cells) {
+  if (cells < 1300000 || !tma_supported(h)) return false;
+  const LayoutParams& L = h->blocks[0].L;
+  const int pad = L.pitch - L.nx, model = h->desc.model;
+  const bool same_warps = 2LL * TMA_CHUNKS * h->sm_count % L.pitch == 0;
+  if (pad == 0) return L.nx >= 96 && (!same_warps || L.pitch % 32 == 0);
+  if (same_warps && (pad <= 3 || L.nx % 2)) return false;
+  const bool short_rows = model == FLB_MODEL_MRT || (model == FLB_MODEL_BGK && pad == 1);
+  return L.nx >= (short_rows ? 128 : 200);
 }
 
 // The step kernel that a handle's shape selects: the staged FP16S kernels

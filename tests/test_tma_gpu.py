@@ -149,10 +149,10 @@ def test_tma_wait_that_gives_up_is_reported_and_the_handle_recovers(gpu_ok):
 
 
 def test_results_of_a_default_handle_report_a_wait_that_gave_up(gpu_ok):
-    """A caller who chose no launch shape runs the bulk-copy kernel at 110^3: until
+    """A caller who chose no launch shape runs the bulk-copy kernel at 128^3: until
     the status is read, every call that brings results to the host reports the
     incomplete step, and uploads, the way back, do not."""
-    lat = F.cavity(108, tau=0.55, storage="fp16s")
+    lat = F.cavity(126, tau=0.55, storage="fp16s")
     assert lat.get_launch() == (4, -2, 4)
     start = lat.download_pops(np.float64)
     lat.set_wait_limit(0.05)
@@ -177,12 +177,23 @@ def test_results_of_a_default_handle_report_a_wait_that_gave_up(gpu_ok):
 
 
 @pytest.mark.parametrize("ni,model,want", [
-    (104, "bgk", (4, 0, 2)),    # 106^3: the last size below the line
+    (99, "bgk", (4, 0, 2)), (100, "bgk", (4, 0, 4)),    # 101^3, 102^3
+    (104, "les", (4, 0, 2)),    # 106^3: the last size below the line
     (106, "bgk", (4, 0, 4)),    # 108^3: above it, rows not on 16-byte boundaries
     (106, "mrt", (4, 0, 2)),
-    (108, "bgk", (4, -2, 4)),   # 110^3: rows of 112
-    (110, "les", (4, -2, 4)),
+    (108, "bgk", (4, 0, 4)),    # 110^3: rows of 112 with two cells of padding
+    (108, "mrt", (4, 0, 4)),
+    (110, "les", (4, -2, 4)),   # 112^3: none
     (110, "mrt", (4, -2, 4)),
+    (118, "bgk", (4, 0, 4)),    # 120^3: the row ends at the same warps of every tile
+    (126, "bgk", (4, -2, 4)),   # 128^3: the same, but in whole warps
+    (158, "mrt", (4, -2, 4)),   # 160^3: in half warps
+    (125, "les", (4, 0, 4)),    # 127^3: with padding
+    (133, "bgk", (4, -2, 4)), (133, "les", (4, 0, 4)), (133, "mrt", (4, -2, 4)),  # 135^3
+    (140, "bgk", (4, 0, 4)), (140, "mrt", (4, -2, 4)),                            # 142^3
+    (131, "les", (4, 0, 4)), (131, "mrt", (4, -2, 4)),                            # 133^3
+    (194, "mrt", (4, 0, 2)), (200, "mrt", (4, 0, 4)),   # 196^3, 202^3
+    (204, "les", (4, -2, 4)),                           # 206^3
 ])
 def test_default_shape_gives_the_direct_kernels_bits(gpu_ok, ni, model, want):
     """The shape the library picks by itself, on both sides of each line of its
@@ -219,7 +230,7 @@ def test_default_shape_follows_the_model_of_a_live_handle(gpu_ok):
 
 
 def test_failed_autotune_leaves_the_default_in_charge(gpu_ok):
-    lat = F.cavity(108, tau=0.55, storage="fp16s", model="mrt")
+    lat = F.cavity(126, tau=0.55, storage="fp16s", model="mrt")
     lat.set_wait_limit(0.05)
     F._capi.call("flb_test_withhold_tile", lat._h, 150)
     lat.step(1)
