@@ -346,6 +346,14 @@ struct Shape {
 // / 13.3).
 bool small_lattice(const HostBlock& b) { return b.padded() <= 300000; }
 
+// Handles whose tile kernel runs its early form: steps short enough for 2 us of launch
+// to weigh more than the spills.  Us a step as usual / early at 64 / 96 / 128 / 160 cells
+// a side in uneven blocks (0.3 / 1.0 / 2.4 / 4.6 M padded cells): FP32 BGK 16.5 / 41.3 /
+// 93.9 / 159.2 and 14.9 / 40.0 / 92.2 / 158.4, two-rate MRT 16.5 / 41.2 / 94.5 / 159.5 and
+// 15.4 / 39.8 / 94.0 / 163.2; FP32S BGK 14.5 / 38.1 / 97.9 / 170.4 and 13.0 / 36.1 / 96.3 /
+// 169.8, LES 18.6 / 48.3 / 118.8 / 208.2 and 16.3 / 46.8 / 118.3 / 209.0.
+bool short_steps(const flb_lattice* h) { return h->dstride <= 3000000; }
+
 // Shape of a handle's steps until flb_set_launch or flb_autotune chooses one.
 // Measured on cavities (us a step at 32 / 64 / 96 / 128 / 192 / 256 / 320 stored
 // cells a side):
@@ -844,8 +852,19 @@ void launch_one_step_v(flb_lattice* h, cudaStream_t st) {
         return;
       }
     }
-    k_pull_blocks<S, R, MODEL, V><<<unsigned(g), dim3(32 * h->tile_y), 0, st>>>(
-        h->sp, h->d_blocks, h->d_tile_block, h->ntiles);
+    // FP64 is no slower in the early form at any size and has it alone
+    constexpr bool always = std::is_same<S, double>::value;
+    if constexpr (TILE_EARLY<S, MODEL>) {
+      if (always || (h->dependent && short_steps(h))) {
+        launch_dependent(h->dependent, k_pull_blocks<S, R, MODEL, V, true>, unsigned(g),
+                         dim3(32 * h->tile_y), 0, st, h->sp, h->d_blocks, h->d_tile_block,
+                         h->ntiles);
+        return;
+      }
+    }
+    if constexpr (!always)
+      k_pull_blocks<S, R, MODEL, V><<<unsigned(g), dim3(32 * h->tile_y), 0, st>>>(
+          h->sp, h->d_blocks, h->d_tile_block, h->ntiles);
   }
 }
 

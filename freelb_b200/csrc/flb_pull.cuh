@@ -30,9 +30,8 @@ namespace flb {
 // for FP32 at 4 cells a thread (200^3: 227 us a step for 220); the tile kernel and
 // the pipeline spill more in FP16S (256^3 in uneven blocks: BGK 447 us for 414, MRT
 // 499 for 472; pipeline MRT 466 for 448).  Those keep the read-only path and are
-// launched as usual, which costs them 2 us a step (64^3 in blocks 16.5 for 14.6).  A
-// form of the tile kernel with ordinary loads for short steps alone rounded FP32 LES
-// differently at 2 cells a thread (other multiply-adds contracted).
+// launched as usual, which costs them 2 us a step; the tile kernel has a form with
+// ordinary loads where that is worth more (TILE_EARLY).
 template <bool RO, typename T>
 __device__ __forceinline__ T load_word(const T* p) {
   if constexpr (RO) return __ldg(p);
@@ -1440,22 +1439,32 @@ __global__ void __launch_bounds__(256, SMALL ? 1 : PullBounds<S, MODEL, V>::min_
   pull_chunk<S, R, MODEL, V, RO, SMALL>(p, g, R(p.omega), 0, x0, y, z);
 }
 
+// Tile kernels that have an early form.  FP16S spills too much in it, and the other
+// FP32 models round differently (other multiply-adds contracted).
+template <typename S, int MODEL>
+constexpr bool TILE_EARLY = std::is_same<S, double>::value || std::is_same<S, dev32>::value ||
+                            (std::is_same<S, float>::value &&
+                             (MODEL == MODEL_BGK || MODEL == MODEL_MRT2));
+
 // Many blocks: tiles of blockDim.x consecutive chunks, numbered block by block
 // (tile_start = first tile of the block, tile_block = block of every tile);
 // CTAs walk the tiles with a grid stride (persistent) or take one tile each.
-// Launched as usual, so its sources are its own alone (load_word); the halo copies
-// after it may start early.
-template <typename S, typename R, int MODEL, int V>
+// Launched as usual, its sources are its own alone (load_word); the halo copies after
+// it may start early.
+//
+// EARLY: the form that may be launched as a dependent, with ordinary loads.
+template <typename S, typename R, int MODEL, int V, bool EARLY = false>
 __global__ void __launch_bounds__(256, PullBounds<S, MODEL, V>::min_ctas)
     k_pull_blocks(const StepParams p, const BlockEntry* __restrict__ blocks,
                   const int* __restrict__ tile_block, long long ntiles) {
   start_dependents();
+  if constexpr (EARLY) wait_prerequisites();
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const BlockEntry& b = blocks[__ldg(tile_block + t)];
     const long long q = (t - b.tile_start) * blockDim.x + threadIdx.x;
     int x0, y, z;
     if (chunk_coords<V>(b.g, q, x0, y, z))
-      pull_chunk<S, R, MODEL, V>(p, b.g, R(b.omega), 0, x0, y, z);
+      pull_chunk<S, R, MODEL, V, !EARLY>(p, b.g, R(b.omega), 0, x0, y, z);
   }
 }
 

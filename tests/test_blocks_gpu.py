@@ -338,3 +338,50 @@ def test_default_shapes_of_many_blocks(gpu_ok, storage, kw, count, want):
         out.append([lat.download_pops(block=k) for k in range(count)])
         lat.close()
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("storage,model,vecs", [
+    ("fp32", "bgk", (2, 4)), ("fp32", "mrt", (2, 4)), ("fp32", "les", (2, 4)),
+    ("fp32", "brinkman", (2, 4)), ("fp32s", "bgk", (2, 4)), ("fp32s", "mrt", (2, 4)),
+    ("fp32s", "les", (2, 4)), ("fp32s", "brinkman", (2, 4)), ("fp64", "bgk", (1, 2)),
+    ("fp64", "mrt", (1, 2)), ("fp64", "les", (1, 2)), ("fp64", "brinkman", (1, 2)),
+])
+def test_early_form_of_the_tile_kernel_gives_the_usual_ones_bits(gpu_ok, storage, model, vecs):
+    """Plain steps of a small handle run the tile kernel's early form, captured ones
+    (a graph's launches are ordered as usual) the other; FP64, which has the early
+    form alone, against the single-block kernel.  Every op, on ragged blocks."""
+    tasks = ((2, "bulk"), (4, "bounceback"), (8, "movingwall"), (16, "field_bgk"))
+    shapes = [(37, 20, 18), (24, 30, 19), (9, 7, 50)]
+    for v in vecs:
+        for ctas in (0, 8):
+            out = []
+            for graph in (False, True):
+                rng = np.random.default_rng(v)
+                lat = F.Lattice.blocks([d + (0, 0, 0) for d in shapes], 0.57,
+                                       mode="independent", storage=storage, model=model,
+                                       tasks=tasks)
+                ones = []
+                for k, d in enumerate(shapes):
+                    n = d[0] * d[1] * d[2]
+                    flags = rng.choice(np.array([1, 2, 4, 8, 16], dtype=np.uint8), size=n,
+                                       p=[.1, .6, .1, .1, .1])
+                    pops = np.repeat(O.W, n) * (1 + 0.05 * rng.standard_normal(19 * n))
+                    u, alpha = 0.03 * rng.standard_normal(3 * n), rng.uniform(0, 1, n)
+                    one = F.Lattice(*d, 0.57, storage=storage, model=model, tasks=tasks)
+                    for to, b in ((lat, k), (one, 0)):
+                        to.upload_flags(flags, block=b)
+                        to.upload_pops(pops, block=b)
+                        to.upload_field("u", u, block=b)
+                        if model == "brinkman":
+                            to.upload_field("alpha", alpha, block=b)
+                    ones.append(one)
+                lat.set_launch(4, ctas, v)
+                lat.step(6, graph=graph)
+                out.append([lat.download_pops(block=k) for k in range(len(shapes))])
+                if storage == "fp64":
+                    for one in ones:
+                        one.set_launch(4, 0, v)
+                        one.step(6)
+                    out.append([one.download_pops() for one in ones])
+            for o in out[1:]:
+                assert all(np.array_equal(a, b) for a, b in zip(out[0], o))
